@@ -35,21 +35,22 @@ namespace zntt {
 
 // Per-field choices, measured on B200 inside the transform's pass kernel
 // (80 registers per thread):
-//   kLazy   4p < 2^256, so butterflies keep values in [0, 2p) (sums below 4p
-//           fit in eight words) and skip the final subtraction of each
-//           product; Q0..Q7 are the limbs of 2p.
+//   kLazy   5.1p < 2^256, so butterflies leave their results unreduced
+//           (shoup.cuh); Q0..Q7 are the limbs of 2p.
 //   kSplit  product form: split accumulators (fe_mul_split) or merged rows
 //           (fe_mul_merged).
+//   kLow64  p = 2^64 - 2^32 + 1 mod 2^64, used by the fixed-factor product.
 //   kScaleCompiled  the pass kernel keeps its output-scaling code in every
 //           pass, also where no pass scales: the register allocation it gets
 //           times faster for this field (B200).
 // The special low limbs of both primes (BN254-Fr: p0 = 2^32 - 2^28 + 1;
-// BLS12-381-Fr: p0 = 1, p1 = 2^32 - 1) allow a reduction from shifts and adds
-// with fewer products.  It times faster alone but slower in the pass kernel,
-// whose register budget its extra live values exceed, so it is not used.
+// BLS12-381-Fr: p0 = 1, p1 = 2^32 - 1) allow a Montgomery reduction from shifts
+// and adds with fewer products.  It times faster alone but slower in the
+// kernels, whose register budget its extra live values exceed, so it is not used.
 struct Bn254Fr {
   static constexpr int kId = 0;
   static constexpr bool kLazy = true;
+  static constexpr bool kLow64 = false;
   static constexpr bool kSplit = false;
   static constexpr bool kScaleCompiled = false;
   static constexpr uint32_t P0 = 0xf0000001u, P1 = 0x43e1f593u, P2 = 0x79b97091u, P3 = 0x2833e848u,
@@ -70,6 +71,7 @@ struct Bn254Fr {
 struct Bls12381Fr {
   static constexpr int kId = 1;
   static constexpr bool kLazy = false;  // 4p > 2^256
+  static constexpr bool kLow64 = true;
   static constexpr bool kSplit = true;
   static constexpr bool kScaleCompiled = true;
   static constexpr uint32_t P0 = 0x00000001u, P1 = 0xffffffffu, P2 = 0xfffe5bfeu, P3 = 0x53bda402u,
@@ -209,29 +211,6 @@ __device__ __forceinline__ fe fe_neg(const fe& a) {
   return fe_sub<F>(z, a);
 }
 
-// p - a for a in [0, p]: the negation of a twiddle factor as a multiplier.  For
-// a != 0 it is -a mod p; for a = 0 it is p, which is not canonical but is a
-// valid left operand of fe_mul (the CIOS bound needs a <= p: the running value
-// stays below 2p) and gives the same reduced product as 0.  One subtraction
-// chain, no select: cheaper than fe_neg on the inverse transform's hot path.
-template <class F>
-__device__ __forceinline__ fe fe_p_minus(const fe& a) {
-  fe r;
-  asm("sub.cc.u32  %0, %8, %16;\n\t"
-      "subc.cc.u32 %1, %9, %17;\n\t"
-      "subc.cc.u32 %2, %10, %18;\n\t"
-      "subc.cc.u32 %3, %11, %19;\n\t"
-      "subc.cc.u32 %4, %12, %20;\n\t"
-      "subc.cc.u32 %5, %13, %21;\n\t"
-      "subc.cc.u32 %6, %14, %22;\n\t"
-      "subc.u32    %7, %15, %23;"
-      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]),
-        "=r"(r.v[7])
-      : "n"(F::P0), "n"(F::P1), "n"(F::P2), "n"(F::P3), "n"(F::P4), "n"(F::P5), "n"(F::P6), "n"(F::P7),
-        "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]));
-  return r;
-}
-
 // x in [0, 2p) -> [0, p): one conditional subtraction of p.
 template <class F>
 __device__ __forceinline__ fe fe_reduce(const fe& x) {
@@ -253,77 +232,6 @@ __device__ __forceinline__ fe fe_reduce(const fe& x) {
   // br == 0xffffffff when x < p: keep x.
   r.v[0] = br ? x.v[0] : d0; r.v[1] = br ? x.v[1] : d1; r.v[2] = br ? x.v[2] : d2; r.v[3] = br ? x.v[3] : d3;
   r.v[4] = br ? x.v[4] : d4; r.v[5] = br ? x.v[5] : d5; r.v[6] = br ? x.v[6] : d6; r.v[7] = br ? x.v[7] : d7;
-  return r;
-}
-
-// Lazy butterfly arithmetic for fields with 4p < 2^256 (F::kLazy): inputs and
-// outputs in [0, 2p).
-// a + b, less 2p when the sum reaches 2p.
-template <class F>
-__device__ __forceinline__ fe fe_add2p(const fe& a, const fe& b) {
-  uint32_t s0, s1, s2, s3, s4, s5, s6, s7;
-  uint32_t d0, d1, d2, d3, d4, d5, d6, d7, br;
-  asm("add.cc.u32  %0, %8, %16;\n\t"
-      "addc.cc.u32 %1, %9, %17;\n\t"
-      "addc.cc.u32 %2, %10, %18;\n\t"
-      "addc.cc.u32 %3, %11, %19;\n\t"
-      "addc.cc.u32 %4, %12, %20;\n\t"
-      "addc.cc.u32 %5, %13, %21;\n\t"
-      "addc.cc.u32 %6, %14, %22;\n\t"
-      "addc.u32    %7, %15, %23;"
-      : "=r"(s0), "=r"(s1), "=r"(s2), "=r"(s3), "=r"(s4), "=r"(s5), "=r"(s6), "=r"(s7)
-      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]),
-        "r"(a.v[7]), "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]),
-        "r"(b.v[6]), "r"(b.v[7]));
-  asm("sub.cc.u32  %0, %9, %17;\n\t"
-      "subc.cc.u32 %1, %10, %18;\n\t"
-      "subc.cc.u32 %2, %11, %19;\n\t"
-      "subc.cc.u32 %3, %12, %20;\n\t"
-      "subc.cc.u32 %4, %13, %21;\n\t"
-      "subc.cc.u32 %5, %14, %22;\n\t"
-      "subc.cc.u32 %6, %15, %23;\n\t"
-      "subc.cc.u32 %7, %16, %24;\n\t"
-      "subc.u32    %8, 0, 0;"
-      : "=r"(d0), "=r"(d1), "=r"(d2), "=r"(d3), "=r"(d4), "=r"(d5), "=r"(d6), "=r"(d7), "=r"(br)
-      : "r"(s0), "r"(s1), "r"(s2), "r"(s3), "r"(s4), "r"(s5), "r"(s6), "r"(s7), "n"(F::Q0),
-        "n"(F::Q1), "n"(F::Q2), "n"(F::Q3), "n"(F::Q4), "n"(F::Q5), "n"(F::Q6), "n"(F::Q7));
-  fe r;
-  r.v[0] = br ? s0 : d0; r.v[1] = br ? s1 : d1; r.v[2] = br ? s2 : d2; r.v[3] = br ? s3 : d3;
-  r.v[4] = br ? s4 : d4; r.v[5] = br ? s5 : d5; r.v[6] = br ? s6 : d6; r.v[7] = br ? s7 : d7;
-  return r;
-}
-
-// a - b, plus 2p when the difference is negative.
-template <class F>
-__device__ __forceinline__ fe fe_sub2p(const fe& a, const fe& b) {
-  uint32_t d0, d1, d2, d3, d4, d5, d6, d7, br;
-  asm("sub.cc.u32  %0, %9, %17;\n\t"
-      "subc.cc.u32 %1, %10, %18;\n\t"
-      "subc.cc.u32 %2, %11, %19;\n\t"
-      "subc.cc.u32 %3, %12, %20;\n\t"
-      "subc.cc.u32 %4, %13, %21;\n\t"
-      "subc.cc.u32 %5, %14, %22;\n\t"
-      "subc.cc.u32 %6, %15, %23;\n\t"
-      "subc.cc.u32 %7, %16, %24;\n\t"
-      "subc.u32    %8, 0, 0;"
-      : "=r"(d0), "=r"(d1), "=r"(d2), "=r"(d3), "=r"(d4), "=r"(d5), "=r"(d6), "=r"(d7), "=r"(br)
-      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]),
-        "r"(a.v[7]), "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]),
-        "r"(b.v[6]), "r"(b.v[7]));
-  fe r;
-  asm("add.cc.u32  %0, %8, %16;\n\t"
-      "addc.cc.u32 %1, %9, %17;\n\t"
-      "addc.cc.u32 %2, %10, %18;\n\t"
-      "addc.cc.u32 %3, %11, %19;\n\t"
-      "addc.cc.u32 %4, %12, %20;\n\t"
-      "addc.cc.u32 %5, %13, %21;\n\t"
-      "addc.cc.u32 %6, %14, %22;\n\t"
-      "addc.u32    %7, %15, %23;"
-      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
-        "=r"(r.v[6]), "=r"(r.v[7])
-      : "r"(d0), "r"(d1), "r"(d2), "r"(d3), "r"(d4), "r"(d5), "r"(d6), "r"(d7), "r"(F::Q0 & br),
-        "r"(F::Q1 & br), "r"(F::Q2 & br), "r"(F::Q3 & br), "r"(F::Q4 & br), "r"(F::Q5 & br),
-        "r"(F::Q6 & br), "r"(F::Q7 & br));
   return r;
 }
 
@@ -439,9 +347,10 @@ __device__ __forceinline__ fe fe_mul_merged(const fe& a, const fe& b) {
 // x * 2^-256 mod p: Montgomery form to the canonical value (REDC of x), the
 // merged-row product with multiplier one but no multiplier products -- eight
 // reduction rows, about half the products of fe_mul.  For x < p the value
-// stays below p + 1, so one conditional subtraction finishes.
+// stays below p + 1, so one conditional subtraction finishes.  `rows`, when
+// given, receives the eight row multipliers, x (-p^-1) mod 2^256.
 template <class F>
-__device__ __forceinline__ fe fe_from_mont(const fe& x) {
+__device__ __forceinline__ fe fe_from_mont(const fe& x, fe* rows = nullptr) {
   uint32_t T[9], U[9];
 #pragma unroll
   for (int q = 0; q < 8; q++) T[q] = x.v[q];
@@ -449,6 +358,7 @@ __device__ __forceinline__ fe fe_from_mont(const fe& x) {
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     const uint32_t m = T[0] * F::N0;
+    if (rows) rows->v[i] = m;
     ZNTT_REDP8(T[0], T[1], T[2], T[3], T[4], T[5], T[6], T[7], T[8], F::P0, F::P2, F::P4, F::P6, m);
     asm("mul.lo.u32 %0, %8, %9;\n\t"
         "mul.hi.u32 %1, %8, %9;\n\t"
@@ -559,15 +469,14 @@ __device__ __forceinline__ fe fe_mul_split(const fe& a, const fe& b) {
 #undef ZNTT_MAD8
 #undef ZNTT_MADP8
 
-// a * b * 2^-256 mod p.  With a < p and b < 2^256 the product is below 2p;
-// kCanon (the default) reduces it to [0, p), as the reference's mul does.
-template <class F, bool kCanon = true>
+// a * b * 2^-256 mod p.  With a < p and b < 2^256 the product is below 2p and is
+// reduced to [0, p), as the reference's mul does.
+template <class F>
 __device__ __forceinline__ fe fe_mul(const fe& a, const fe& b) {
   fe r;
   if constexpr (F::kSplit) r = fe_mul_split<F>(a, b);
   else r = fe_mul_merged<F>(a, b);
-  if constexpr (kCanon) r = fe_reduce<F>(r);
-  return r;
+  return fe_reduce<F>(r);
 }
 
 // Global-memory element access: an element is 32 bytes = two uint4.

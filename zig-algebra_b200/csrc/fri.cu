@@ -56,7 +56,7 @@ int powers_device(int field, const uint64_t* base, const uint64_t* c, uint4* out
   int rc = pool_get(pw.size() * 8, &d_pw);
   if (rc) return rc;
   cudaError_t ce = cudaMemcpyAsync(d_pw, pw.data(), pw.size() * 8, cudaMemcpyHostToDevice, st);
-  if (ce == cudaSuccess) ce = launch_powers(field, (const uint4*)d_pw, c, out, count, st);
+  if (ce == cudaSuccess) ce = launch_powers(field, (const uint4*)d_pw, c, out, count, false, st);
   cudaError_t ce2 = cudaStreamSynchronize(st);  // the power tables return to the pool
   pool_put(d_pw, pw.size() * 8);
   if (ce == cudaSuccess) ce = ce2;

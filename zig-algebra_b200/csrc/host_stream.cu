@@ -37,8 +37,6 @@ extern "C" int zntt_ntt_host_many(const zntt_twiddles* tw, uint64_t* const* h_da
   const uint32_t log_n = e->log_n;
   const size_t bytes = (size_t)32 << log_n;
   const bool inverse = mode == ZNTT_INVERSE;
-  uint64_t ninv[4];
-  if (inverse) n_inverse(e->field, log_n, ninv);
   const Plan plan = tuned_plan(e->field, log_n);
   const int depth = (int)std::min<size_t>(kDepth, count);
   void* a[kDepth] = {nullptr, nullptr, nullptr};
@@ -58,7 +56,7 @@ extern "C" int zntt_ntt_host_many(const zntt_twiddles* tw, uint64_t* const* h_da
     cudaStream_t st = c.pipe[d];
     ce = cudaMemcpyAsync(a[d], h_data[i], bytes, cudaMemcpyHostToDevice, st);
     if (ce != cudaSuccess) break;
-    rc = run_plan(e->field, e, plan, log_n, (const uint4*)a[d], (uint4*)b[d], nullptr, inverse, inverse, ninv, st);
+    rc = run_plan(e->field, e, plan, log_n, (const uint4*)a[d], (uint4*)b[d], nullptr, inverse, inverse, st);
     if (rc) break;
     ce = cudaMemcpyAsync(h_data[i], b[d], bytes, cudaMemcpyDeviceToHost, st);
   }

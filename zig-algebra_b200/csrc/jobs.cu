@@ -39,7 +39,7 @@ int acquire_coset_tab(int field, uint32_t log_in, const uint64_t* shift, CosetTa
   t->field = field;
   t->log_in = log_in;
   std::memcpy(t->shift, shift, 32);
-  t->bytes = ((size_t)32) << log_in;
+  t->bytes = ((size_t)64) << log_in;
   cudaError_t ce = cudaMalloc((void**)&t->d, t->bytes);
   if (ce != cudaSuccess) {
     delete t;
@@ -57,7 +57,7 @@ int acquire_coset_tab(int field, uint32_t log_in, const uint64_t* shift, CosetTa
     return rc;
   }
   ce = cudaMemcpyAsync(d_pw, pw.data(), pw.size() * 8, cudaMemcpyHostToDevice, st);
-  if (ce == cudaSuccess) ce = launch_powers(field, (const uint4*)d_pw, ninv, t->d, 1ull << log_in, st);
+  if (ce == cudaSuccess) ce = launch_powers(field, (const uint4*)d_pw, ninv, t->d, 1ull << log_in, true, st);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
   pool_put(d_pw, pw.size() * 8);
   if (ce != cudaSuccess) {
@@ -94,6 +94,7 @@ static PassParams pass_params(const TwEntry* tw, uint32_t log_n, const PassDesc&
   pp.src = src;
   pp.dst = dst;
   pp.tw = tw->d_table;
+  pp.wide = pass_wide(src, dst);
   pp.log_n = log_n;
   pp.S = d.S;
   pp.k = d.k;
@@ -120,16 +121,15 @@ Plan batch_plan(int field, uint32_t log_n, int shape) {
 // Appends the passes of one transform src -> dst (mid: where passes after the
 // first run in place).
 void plan_transform(JobPlan& jp, const TwEntry* tw, const Plan& plan, uint32_t log_n, const uint4* src,
-                           uint4* mid, uint4* dst, bool inverse, const uint64_t* scale_val, const uint4* scale_tab,
+                           uint4* mid, uint4* dst, bool inverse, ScaleKind scale, const uint4* scale_tab,
                            uint64_t src_len, uint64_t dst_len) {
   for (uint32_t p = 0; p < plan.np; p++) {
     const bool first = p == 0, last = p + 1 == plan.np;
     PassParams pp = pass_params(tw, log_n, plan.p[p], first, inverse, first ? src : mid, last ? dst : mid);
     if (first) pp.src_len = src_len;
     if (last) pp.dst_len = dst_len;
-    if (last && (scale_val || scale_tab)) {
-      pp.scale = 1;
-      if (scale_val) std::memcpy(pp.scale_val, scale_val, 32);
+    if (last) {
+      pp.scale = scale;
       pp.scale_tab = scale_tab;
     }
     jp.passes.push_back(pp);
@@ -148,11 +148,9 @@ void plan_poly_mul(JobPlan& jp, const TwEntry* tw, const Plan& plan, const uint4
                    uint64_t len_b, uint4* s1, uint4* s2, uint4* dst) {
   const uint32_t L = tw->log_n;
   const uint64_t n = 1ull << L;
-  uint64_t ninv[4];
-  n_inverse(tw->field, L, ninv);
-  plan_transform(jp, tw, plan, L, a, s1, s1, false, nullptr, nullptr, len_a, n);
-  plan_transform(jp, tw, plan, L, b, s2, s2, false, nullptr, s1, len_b, n);
-  plan_transform(jp, tw, plan, L, s2, s1, dst, true, ninv, nullptr, n, len_a + len_b - 1);
+  plan_transform(jp, tw, plan, L, a, s1, s1, false, kScaleNone, nullptr, len_a, n);
+  plan_transform(jp, tw, plan, L, b, s2, s2, false, kScaleElements, s1, len_b, n);
+  plan_transform(jp, tw, plan, L, s2, s1, dst, true, kScaleFixed, tw->n_inv(), n, len_a + len_b - 1);
 }
 
 }  // namespace zntt
@@ -251,10 +249,9 @@ int zntt_batch_create(int field, const zntt_job* jobs, size_t n_jobs, int shape,
         b->scratch.push_back({s, (size_t)32 << L});
         mid = (uint4*)s;
       }
-      uint64_t ninv[4];
       const bool inv = job.mode == ZNTT_INVERSE;
-      if (inv) n_inverse(field, L, ninv);
-      plan_transform(plans[j], tw, plan, L, src, mid, dst, inv, inv ? ninv : nullptr, nullptr, 1ull << L, 1ull << L);
+      plan_transform(plans[j], tw, plan, L, src, mid, dst, inv, inv ? kScaleFixed : kScaleNone, tw->n_inv(), 1ull << L,
+                     1ull << L);
     } else if (job.kind == ZNTT_JOB_POLY_MUL) {
       void* s1 = nullptr;
       void* s2 = nullptr;
@@ -289,9 +286,9 @@ int zntt_batch_create(int field, const zntt_job* jobs, size_t n_jobs, int shape,
       b->scratch.push_back({coef, (size_t)32 << Li});
       const Plan pin = batch_plan(field, Li, b->shape);
       const Plan pout = batch_plan(field, L, b->shape);
-      plan_transform(plans[j], twi, pin, Li, src, (uint4*)coef, (uint4*)coef, true, nullptr, ct->d, 1ull << Li,
+      plan_transform(plans[j], twi, pin, Li, src, (uint4*)coef, (uint4*)coef, true, kScaleFixedTab, ct->d, 1ull << Li,
                      1ull << Li);
-      plan_transform(plans[j], tw, pout, L, (const uint4*)coef, dst, dst, false, nullptr, nullptr, 1ull << Li,
+      plan_transform(plans[j], tw, pout, L, (const uint4*)coef, dst, dst, false, kScaleNone, nullptr, 1ull << Li,
                      1ull << L);
     }
   }
@@ -464,9 +461,9 @@ int zntt_coset_lde_device(const zntt_twiddles* tw_in, const zntt_twiddles* tw_ou
   JobPlan jp;
   const Plan pin = tuned_plan(ti->field, ti->log_n);
   const Plan pout = tuned_plan(to->field, to->log_n);
-  plan_transform(jp, ti, pin, ti->log_n, (const uint4*)d_evals, (uint4*)coef, (uint4*)coef, true, nullptr, ct->d,
+  plan_transform(jp, ti, pin, ti->log_n, (const uint4*)d_evals, (uint4*)coef, (uint4*)coef, true, kScaleFixedTab, ct->d,
                  1ull << ti->log_n, 1ull << ti->log_n);
-  plan_transform(jp, to, pout, to->log_n, (const uint4*)coef, (uint4*)d_out, (uint4*)d_out, false, nullptr, nullptr,
+  plan_transform(jp, to, pout, to->log_n, (const uint4*)coef, (uint4*)d_out, (uint4*)d_out, false, kScaleNone, nullptr,
                  1ull << ti->log_n, 1ull << to->log_n);
   cudaError_t ce = cudaSuccess;
   for (size_t p = 0; p < jp.passes.size() && ce == cudaSuccess; p++) {
@@ -530,8 +527,6 @@ int zntt_autotune(int field, uint32_t log_n_min, uint32_t log_n_max) {
     if (!rc) rc = pool_get((size_t)32 << L, &y);
     uint8_t seed[32] = {7};
     if (!rc) rc = zntt_random_elements(field, seed, (uint64_t*)x, (size_t)1 << L, nullptr);
-    uint64_t ninv[4];
-    n_inverse(field, L, ninv);
     for (int sh = 0; sh < kNumShapes && !rc; sh++) {
       const uint32_t lt = kShapes[sh].log_tile;
       TuneEntry best;
@@ -545,8 +540,8 @@ int zntt_autotune(int field, uint32_t log_n_min, uint32_t log_n_max) {
         // Each repetition is a forward and an inverse transform (the inverse's
         // last pass also scales by 1/n): one plan serves both directions.
         auto both = [&]() {
-          int r2 = run_plan(field, tw, plan, L, (const uint4*)x, (uint4*)y, nullptr, false, false, nullptr, st);
-          if (!r2) r2 = run_plan(field, tw, plan, L, (const uint4*)x, (uint4*)y, nullptr, true, true, ninv, st);
+          int r2 = run_plan(field, tw, plan, L, (const uint4*)x, (uint4*)y, nullptr, false, false, st);
+          if (!r2) r2 = run_plan(field, tw, plan, L, (const uint4*)x, (uint4*)y, nullptr, true, true, st);
           return r2;
         };
         for (int w = 0; w < 2 && !rc; w++) rc = both();

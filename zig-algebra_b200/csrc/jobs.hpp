@@ -8,7 +8,7 @@
 
 namespace zntt {
 
-// n^-1 * g^i for i < 2^log_in, cached per (field, log_in, g) and reference counted.
+// n^-1 * g^i for i < 2^log_in as fixed factors (shoup.cuh), cached per (field, log_in, g) and reference counted.
 struct CosetTab {
   int field = 0;
   uint32_t log_in = 0;
@@ -32,11 +32,11 @@ struct JobPlan {
 Plan batch_plan(int field, uint32_t log_n, int shape);
 
 // Appends the passes of one transform src -> dst (mid: where passes after the
-// first run in place); the last pass scales by scale_val or scale_tab when
-// given and stores only the output positions below dst_len; the first pass
+// first run in place); the last pass scales by `scale` (with the factor or table
+// scale_tab) and stores only the output positions below dst_len; the first pass
 // reads zeros from input index src_len on.
 void plan_transform(JobPlan& jp, const TwEntry* tw, const Plan& plan, uint32_t log_n, const uint4* src, uint4* mid,
-                    uint4* dst, bool inverse, const uint64_t* scale_val, const uint4* scale_tab, uint64_t src_len,
+                    uint4* dst, bool inverse, ScaleKind scale, const uint4* scale_tab, uint64_t src_len,
                     uint64_t dst_len);
 
 // The passes of one polynomial product (ZNTT_JOB_POLY_MUL) on 2^log_n points:

@@ -5,6 +5,7 @@
 // stages a tile of the vector in shared memory with coalesced 16-byte global
 // loads, runs several butterfly stages on it, and writes it back.  All
 // arithmetic is exact Montgomery arithmetic from field.cuh.
+#include <algorithm>
 #include <cstring>
 
 #include "field.cuh"
@@ -101,57 +102,111 @@ cudaError_t launch_ntt_pass(int field, int shape, const PassParams& pp, uint64_t
 // Twiddle table
 // ---------------------------------------------------------------------------
 
+static int grid_for(uint64_t count) { return (int)std::min<uint64_t>((count + 255) / 256, 148 * 16); }
+
 template <class F>
-__global__ void twiddle_table_kernel(const uint4* __restrict__ pw, uint4* __restrict__ table, uint32_t log_n) {
-  const uint64_t total = (1ull << log_n) - 1;
+__global__ void twiddle_table_kernel(const uint4* __restrict__ pw, fe n_inv, uint4* __restrict__ table,
+                                     uint32_t log_n) {
+  const uint64_t total = 1ull << log_n;
   for (uint64_t f = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; f < total;
        f += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t s = 63 - __clzll(f + 1);           // stage: 2^s - 1 <= f < 2^(s+1) - 1
-    const uint64_t j = f + 1 - (1ull << s);
-    const uint64_t e = j << (log_n - 1 - s);           // exponent of root, < 2^(log_n-1)
-    const uint32_t e0 = e & 1023, e1 = (e >> 10) & 1023, e2 = (uint32_t)(e >> 20);
-    fe r = fe_mul<F>(fe_load_nc(pw + 2 * e0), fe_load_nc(pw + 2 * (1024 + e1)));
-    r = fe_mul<F>(r, fe_load_nc(pw + 2 * (2048 + e2)));
-    fe_store(table + 2 * f, r);
+    fe r = n_inv;
+    if (f + 1 < total) {
+      const uint32_t s = 63 - __clzll(f + 1);           // stage: 2^s - 1 <= f < 2^(s+1) - 1
+      const uint64_t j = f + 1 - (1ull << s);
+      const uint64_t e = j << (log_n - 1 - s);           // exponent of root, < 2^(log_n-1)
+      const uint32_t e0 = e & 1023, e1 = (e >> 10) & 1023, e2 = (uint32_t)(e >> 20);
+      r = fe_mul<F>(fe_load_nc(pw + 2 * e0), fe_load_nc(pw + 2 * (1024 + e1)));
+      r = fe_mul<F>(r, fe_load_nc(pw + 2 * (2048 + e2)));
+    }
+    pair_store(table + 4 * f, pair_of<F>(r));
   }
 }
 
-cudaError_t launch_twiddle_table(int field, const uint4* d_pw, uint4* d_table, uint32_t log_n, cudaStream_t st) {
-  if (log_n == 0) return cudaSuccess;
-  const uint64_t total = (1ull << log_n) - 1;
-  uint64_t blocks = (total + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
+cudaError_t launch_twiddle_table(int field, const uint4* d_pw, const uint64_t* n_inv, uint4* d_table, uint32_t log_n,
+                                 cudaStream_t st) {
+  fe ni;
+  std::memcpy(ni.v, n_inv, 32);
+  const int blocks = grid_for(1ull << log_n);
   if (field == kBn254Fr)
-    twiddle_table_kernel<Bn254Fr><<<(unsigned)blocks, 256, 0, st>>>(d_pw, d_table, log_n);
+    twiddle_table_kernel<Bn254Fr><<<blocks, 256, 0, st>>>(d_pw, ni, d_table, log_n);
   else
-    twiddle_table_kernel<Bls12381Fr><<<(unsigned)blocks, 256, 0, st>>>(d_pw, d_table, log_n);
+    twiddle_table_kernel<Bls12381Fr><<<blocks, 256, 0, st>>>(d_pw, ni, d_table, log_n);
+  return cudaGetLastError();
+}
+
+// A caller's entries may be any 256-bit values: they are reduced first.
+template <class F>
+__global__ void twiddle_pairs_kernel(const uint4* __restrict__ entries, fe n_inv, uint4* __restrict__ table,
+                                     uint32_t log_n) {
+  const uint64_t total = 1ull << log_n;
+  for (uint64_t f = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; f < total;
+       f += (uint64_t)gridDim.x * blockDim.x) {
+    fe r = n_inv;
+    if (f + 1 < total) {
+      r = fe_load_nc(entries + 2 * f);
+      for (int k = 0; k < 6 && !fe_lt_p<F>(r); k++) r = fe_reduce<F>(r);
+    }
+    pair_store(table + 4 * f, pair_of<F>(r));
+  }
+}
+
+cudaError_t launch_twiddle_pairs(int field, const uint4* d_entries, const uint64_t* n_inv, uint4* d_table,
+                                 uint32_t log_n, cudaStream_t st) {
+  fe ni;
+  std::memcpy(ni.v, n_inv, 32);
+  const int blocks = grid_for(1ull << log_n);
+  if (field == kBn254Fr)
+    twiddle_pairs_kernel<Bn254Fr><<<blocks, 256, 0, st>>>(d_entries, ni, d_table, log_n);
+  else
+    twiddle_pairs_kernel<Bls12381Fr><<<blocks, 256, 0, st>>>(d_entries, ni, d_table, log_n);
+  return cudaGetLastError();
+}
+
+template <class F>
+__global__ void pair_entries_kernel(const uint4* __restrict__ pairs, uint4* __restrict__ entries, uint64_t count) {
+  for (uint64_t f = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; f < count;
+       f += (uint64_t)gridDim.x * blockDim.x)
+    fe_store(entries + 2 * f, pair_entry<F>(ld_fe32(pairs + 4 * f + 2)));
+}
+
+cudaError_t launch_pair_entries(int field, const uint4* d_pairs, uint4* d_entries, uint64_t count, cudaStream_t st) {
+  if (count == 0) return cudaSuccess;
+  if (field == kBn254Fr)
+    pair_entries_kernel<Bn254Fr><<<grid_for(count), 256, 0, st>>>(d_pairs, d_entries, count);
+  else
+    pair_entries_kernel<Bls12381Fr><<<grid_for(count), 256, 0, st>>>(d_pairs, d_entries, count);
   return cudaGetLastError();
 }
 
 // out[i] = c * base^i from three host-made power tables of the base
 // (pw[0][i] = base^i, pw[1][i] = base^(1024 i), pw[2][i] = base^(2^20 i)).
-template <class F>
+template <class F, bool PAIRS>
 __global__ void powers_kernel(const uint4* __restrict__ pw, fe c, uint4* __restrict__ out, uint64_t count) {
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < count;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t e0 = i & 1023, e1 = (i >> 10) & 1023, e2 = (uint32_t)(i >> 20);
     fe r = fe_mul<F>(fe_load_nc(pw + 2 * e0), fe_load_nc(pw + 2 * (1024 + e1)));
     r = fe_mul<F>(r, fe_load_nc(pw + 2 * (2048 + e2)));
-    fe_store(out + 2 * i, fe_mul<F>(r, c));
+    r = fe_mul<F>(r, c);
+    if constexpr (PAIRS) pair_store(out + 4 * i, pair_of<F>(r));
+    else fe_store(out + 2 * i, r);
   }
 }
 
-cudaError_t launch_powers(int field, const uint4* d_pw, const uint64_t* c, uint4* out, uint64_t count,
+cudaError_t launch_powers(int field, const uint4* d_pw, const uint64_t* c, uint4* out, uint64_t count, bool pairs,
                           cudaStream_t st) {
   fe cv;
   std::memcpy(cv.v, c, 32);
-  uint64_t blocks = (count + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  if (blocks == 0) return cudaSuccess;
-  if (field == kBn254Fr)
-    powers_kernel<Bn254Fr><<<(unsigned)blocks, 256, 0, st>>>(d_pw, cv, out, count);
-  else
-    powers_kernel<Bls12381Fr><<<(unsigned)blocks, 256, 0, st>>>(d_pw, cv, out, count);
+  if (count == 0) return cudaSuccess;
+  const int blocks = grid_for(count);
+  if (field == kBn254Fr) {
+    if (pairs) powers_kernel<Bn254Fr, true><<<blocks, 256, 0, st>>>(d_pw, cv, out, count);
+    else powers_kernel<Bn254Fr, false><<<blocks, 256, 0, st>>>(d_pw, cv, out, count);
+  } else {
+    if (pairs) powers_kernel<Bls12381Fr, true><<<blocks, 256, 0, st>>>(d_pw, cv, out, count);
+    else powers_kernel<Bls12381Fr, false><<<blocks, 256, 0, st>>>(d_pw, cv, out, count);
+  }
   return cudaGetLastError();
 }
 

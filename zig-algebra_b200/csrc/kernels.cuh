@@ -11,6 +11,11 @@ namespace zntt {
 // 2 and 3: SmallField's Goldilocks and BabyBear (8-byte elements, small.cu).
 enum FieldId : int { kBn254Fr = 0, kBls12381Fr = 1, kGoldilocksField = 2, kBabyBearField = 3 };
 
+// The output scaling of a pass: none, one fixed factor (the inverse's 1/n), a
+// table of fixed factors (a coset extension's n^-1 g^q), or a table of elements
+// (the other transform of a polynomial product).
+enum ScaleKind : uint32_t { kScaleNone = 0, kScaleFixed = 1, kScaleFixedTab = 2, kScaleElements = 3 };
+
 // One fused radix-2^k pass of the decimation-in-time network.
 //
 // The network is zig-ntt's (libs/ntt/src/root.zig:148-212): bit-reverse the
@@ -25,17 +30,17 @@ enum FieldId : int { kBn254Fr = 0, kBls12381Fr = 1, kGoldilocksField = 2, kBabyB
 struct PassParams {
   const uint4* src;   // 2 uint4 per element
   uint4* dst;
-  const uint4* tw;    // zig-ntt twiddle table, stage s at entry 2^s - 1
+  const uint4* tw;    // zig-ntt twiddle table as fixed factors (shoup.cuh), 4 uint4 each, stage s at entry 2^s - 1
   uint32_t log_n;     // L
   uint32_t S;         // stages already applied
   uint32_t k;         // stages in this pass
   uint32_t c;         // log2 of contiguous positions per tile row
   uint32_t first;     // gather the input through the bit reversal
   uint32_t inverse;   // inttWithTwiddles mapping: w = 1 (j = 0) or -tw[s-1][2^(s-1) - j]
+  uint32_t wide;      // src and dst are 32-byte aligned
   uint32_t tw0_one;   // every stage's entry 0 is one (j = 0 needs no multiply)
-  uint32_t scale;     // multiply each output by scale_val (or scale_tab[q]) after the last stage
-  uint32_t scale_val[8];
-  const uint4* scale_tab;  // when non-null, output position q is scaled by scale_tab[q]
+  uint32_t scale;     // what the outputs are multiplied by after the last stage (ScaleKind)
+  const uint4* scale_tab;  // the factor, or the table whose entry q multiplies output position q
   uint64_t src_len;   // first pass: natural input index >= src_len reads as zero (zero padding)
   uint64_t dst_len;   // output positions >= dst_len are not stored
 };
@@ -70,7 +75,12 @@ inline int shape_smem_bytes(int shape) { return (1 << kShapes[shape].log_tile) *
 // of its output runs the extension variant of the kernels.
 inline bool pass_needs_ext(const PassParams& pp) {
   const uint64_t n = 1ull << pp.log_n;
-  return (pp.first && pp.src_len < n) || (pp.scale && pp.scale_tab != nullptr) || pp.dst_len < n;
+  return (pp.first && pp.src_len < n) || pp.scale >= kScaleFixedTab || pp.dst_len < n;
+}
+
+// PassParams::wide of a pass between the two vectors.
+inline uint32_t pass_wide(const uint4* src, const uint4* dst) {
+  return ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 31) == 0;
 }
 
 cudaError_t launch_ntt_pass(int field, int shape, const PassParams& pp, uint64_t num_tiles, cudaStream_t st);
@@ -103,16 +113,22 @@ inline bool batch_all_full(int shape, const BatchPass* passes, size_t n) {
 }
 int batch_grid(int field, int shape, bool ext);
 
-// Flat zig-ntt twiddle table for one (field, log_n, root): entry 2^s - 1 + j
-// of stage s is root^(j * 2^(log_n-1-s)).  The powers are assembled from three
+// Flat zig-ntt twiddle table for one (field, log_n, root), as fixed factors:
+// entry 2^s - 1 + j of stage s is root^(j * 2^(log_n-1-s)), and the last entry
+// (2^log_n - 1) is 1/n, given in Montgomery form.  The powers are assembled from three
 // small host-made tables: pw[0][i] = root^i, pw[1][i] = root^(1024 i),
 // pw[2][i] = root^(2^20 i), i < 1024 (each 1024 x 32 bytes, contiguous).
-cudaError_t launch_twiddle_table(int field, const uint4* d_pw, uint4* d_table, uint32_t log_n,
+cudaError_t launch_twiddle_table(int field, const uint4* d_pw, const uint64_t* n_inv, uint4* d_table, uint32_t log_n,
                                  cudaStream_t st);
+// The same from the table's 2^log_n - 1 entries in Montgomery form.
+cudaError_t launch_twiddle_pairs(int field, const uint4* d_entries, const uint64_t* n_inv, uint4* d_table,
+                                 uint32_t log_n, cudaStream_t st);
+// `count` fixed factors from d_pairs on, back in Montgomery form.
+cudaError_t launch_pair_entries(int field, const uint4* d_pairs, uint4* d_entries, uint64_t count, cudaStream_t st);
 
 // out[i] = c * base^i for i < count (count <= 2^30), from the three power
-// tables of `base` laid out as for launch_twiddle_table.
-cudaError_t launch_powers(int field, const uint4* d_pw, const uint64_t* c, uint4* out, uint64_t count,
+// tables of `base` laid out as for launch_twiddle_table; `pairs`: as fixed factors.
+cudaError_t launch_powers(int field, const uint4* d_pw, const uint64_t* c, uint4* out, uint64_t count, bool pairs,
                           cudaStream_t st);
 
 // dst[rev(i)] = src[i] for 2^log_n elements (out of place).

@@ -91,14 +91,7 @@ extern "C" int zntt_ntt_device_inplace_noalloc(const zntt_twiddles* tw, uint64_t
   const uint32_t np = plan.np;
   const PassDesc* passes = plan.p;
 
-  uint64_t ninv[4] = {0, 0, 0, 0};
   const bool inverse = mode == ZNTT_INVERSE;
-  if (inverse) {
-    const HostField& F = host_field(e->field);
-    uint64_t nf[4];
-    F.from_u64((uint64_t)1 << log_n, nf);
-    F.inv(nf, ninv);
-  }
   cudaStream_t st = stream ? (cudaStream_t)stream : c.stream;
   uint4* data = reinterpret_cast<uint4*>(d_data);
   for (uint32_t p = 0; p < np; p++) {
@@ -110,6 +103,7 @@ extern "C" int zntt_ntt_device_inplace_noalloc(const zntt_twiddles* tw, uint64_t
     pp.src = first ? data : scratch;
     pp.dst = (np == 1 || last) ? data : scratch;
     pp.tw = e->d_table;
+    pp.wide = pass_wide(pp.src, pp.dst);
     pp.log_n = log_n;
     pp.S = passes[p].S;
     pp.k = passes[p].k;
@@ -117,8 +111,8 @@ extern "C" int zntt_ntt_device_inplace_noalloc(const zntt_twiddles* tw, uint64_t
     pp.first = first;
     pp.inverse = inverse;
     pp.tw0_one = e->tw0_one;
-    pp.scale = last && inverse;
-    if (pp.scale) std::memcpy(pp.scale_val, ninv, 32);
+    pp.scale = last && inverse ? kScaleFixed : kScaleNone;
+    pp.scale_tab = e->n_inv();
     pp.src_len = 1ull << log_n;
     pp.dst_len = 1ull << log_n;
     const uint64_t tiles = (1ull << log_n) >> (pp.k + pp.c);

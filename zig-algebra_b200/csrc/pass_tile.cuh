@@ -11,6 +11,7 @@
 
 #include "field.cuh"
 #include "kernels.cuh"
+#include "shoup.cuh"
 
 namespace zntt {
 
@@ -32,53 +33,56 @@ __device__ __forceinline__ void sm_store(uint4* sm, uint32_t e, const fe& a) {
   sm[TILE + e] = make_uint4(a.v[4], a.v[5], a.v[6], a.v[7]);
 }
 
-// Twiddle of global stage s (1-based) for butterfly index jg, with the
-// forward (tw[s-1][jg]) or inttWithTwiddles (1 or -tw[s-1][2^(s-1) - jg])
-// mapping.  `stw` points at tw[s-1]; returns false when the factor is one and
-// the multiply can be skipped (unit0: entry 0 is one, always so for the inverse).  The inverse's factor is p - tw (fe_p_minus):
-// the product equals the one by -tw mod p, also for a zero entry.
+// t = w v for the table entry `idx` of a stage (mul), or v itself: below 2 p for
+// lazy fields, below p for the others.
 template <class F>
-__device__ __forceinline__ bool twiddle(bool inverse, bool unit0, const uint4* stw, uint32_t half_g, uint32_t jg,
-                                        fe& w) {
-  if (jg == 0 && unit0) return false;
-  if (!inverse) {
-    w = fe_load_nc(stw + (jg << 1));
-  } else {
-    w = fe_p_minus<F>(fe_load_nc(stw + ((half_g - jg) << 1)));
-  }
-  return true;
+__device__ __forceinline__ fe times_factor(bool mul, const uint4* stw, uint32_t idx, const fe& v) {
+  if (!mul) return fe_weak<F>(v);
+  const uint4* f = stw + 4ull * idx;
+  const fe t = fe_mul_fixed<F>(v, ld_fe32(f), ld_fe32(f + 2));
+  if constexpr (F::kLazy) return t;
+  else return fe_reduce<F>(t);
 }
 
-// u, v -> u + w v, u - w v.  Lazy fields (4p < 2^256) keep u and v in
-// [0, 2p) between stages; the last stage of a pass reduces them to [0, p), so
-// every pass reads and writes canonical elements.
-template <class F>
-__device__ __forceinline__ void butterfly(fe& u, fe& v, bool mul, const fe& w) {
-  if constexpr (F::kLazy) {
-    const fe t = mul ? fe_mul<F, false>(w, v) : v;
-    v = fe_sub2p<F>(u, t);
-    u = fe_add2p<F>(u, t);
-  } else {
-    const fe t = mul ? fe_mul<F>(w, v) : v;
-    v = fe_sub<F>(u, t);
-    u = fe_add<F>(u, t);
-  }
-}
-
-// [0, 2p) -> [0, p) after a pass's last stage (lazy fields only).
-template <class F>
-__device__ __forceinline__ void canonical(fe& x, bool last) {
-  if constexpr (F::kLazy) {
-    if (last) x = fe_reduce<F>(x);
-  }
-}
-
-// Global loads of tile data: COHERENT reads through L2 only, for data other
-// SMs wrote earlier in the same launch (the batched kernel).
+// Global access to tile data, one element (32 bytes) per thread.  `wide`: the
+// vectors are 32-byte aligned, and an element moves in one instruction; else in
+// two of 16 bytes.  COHERENT reads through L2 only, for data other SMs wrote
+// earlier in the same launch (the batched kernel).
 template <bool COHERENT>
-__device__ __forceinline__ uint4 load_data(const uint4* p) {
-  if constexpr (COHERENT) return __ldcg(p);
-  else return *p;
+__device__ __forceinline__ fe load_data(const uint4* p, bool wide) {
+  fe r;
+  if (wide) {
+    if constexpr (COHERENT)
+      asm volatile("ld.global.cg.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                   : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]),
+                     "=r"(r.v[7])
+                   : "l"(p));
+    else
+      asm volatile("ld.global.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                   : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]),
+                     "=r"(r.v[7])
+                   : "l"(p));
+    return r;
+  }
+  uint4 lo, hi;
+  if constexpr (COHERENT) {
+    lo = __ldcg(p);
+    hi = __ldcg(p + 1);
+  } else {
+    lo = p[0];
+    hi = p[1];
+  }
+  r.v[0] = lo.x; r.v[1] = lo.y; r.v[2] = lo.z; r.v[3] = lo.w;
+  r.v[4] = hi.x; r.v[5] = hi.y; r.v[6] = hi.z; r.v[7] = hi.w;
+  return r;
+}
+__device__ __forceinline__ void store_data(uint4* p, const fe& a, bool wide) {
+  if (wide)
+    asm volatile("st.global.v8.u32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.v[0]), "r"(a.v[1]),
+                 "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7])
+                 : "memory");
+  else
+    fe_store(p, a);
 }
 
 // EXT enables the extension features: zero padding of the first pass's input
@@ -90,177 +94,238 @@ __device__ __forceinline__ uint4 load_data(const uint4* p) {
 // (2^24 BN254-Fr, B200).  SCALE compiles the output scaling (the inverse's
 // 1/n, the extension's factor table); a pass launched without it must not ask
 // for scaling (pp.scale == 0).
+//
+// The first stages read their elements straight from global memory and the last
+// ones write theirs there (an element is one 32-byte sector, so a thread's own
+// element moves as efficiently as a coalesced row); shared memory only carries
+// the exchanges between stage pairs.
 template <class F, int LOG_TILE, int THREADS, bool COHERENT, bool EXT, bool FULL = false, bool SCALE = true>
-__device__ __forceinline__ void ntt_tile(const PassParams& pp, uint64_t blk, uint4* sm) {
-  constexpr uint32_t TILE_MAX = 1u << LOG_TILE;
+struct TilePass {
+  static constexpr uint32_t TILE_MAX = 1u << LOG_TILE;
+  const PassParams& pp;
+  uint4* const sm;
   // The fields the stage loop reads, read once (for parameters held in
   // memory rather than in the kernel's parameter space, each later read would
   // be a load re-issued after every barrier).
-  const uint32_t k = pp.k, c = pp.c, C = 1u << c, S = pp.S;
-  const bool first = pp.first, inverse = pp.inverse, unit0 = pp.inverse | pp.tw0_one;
-  const uint4* const tw = pp.tw;
-  const uint32_t tile = FULL ? TILE_MAX : 1u << (k + c);
-  const uint32_t tid = threadIdx.x;
-
+  const uint32_t k, c, C, S;
+  const bool first, inverse, unit0, wide;
+  const uint4* const tw;
   // Indices fit 32 bits: transforms and tables hold at most 2^31 elements, so
   // an element's 16-byte-half offset is below 2^32.
-  const uint32_t b = (uint32_t)blk;
   uint32_t hi_base = 0, m0 = 0, col0 = 0;
-  if (first) {
-    col0 = b << c;
-  } else {
-    const uint32_t mlog = S - c;
-    hi_base = (b >> mlog) << (S + k);
-    m0 = (b & ((1u << mlog) - 1)) << c;
-  }
-  const uint32_t xcols_log = pp.log_n - k;
-  const uint64_t src_len = pp.src_len;
 
-  // ---- load: warp w stages the 128-element slices w, w + W, w + 2W, ... of
-  // the tile (DIT order), column-fastest in 16-byte halves.  These are the
-  // elements its radix-4 groups use while a group's span, 4 h C elements, stays
-  // within 128: those stage pairs exchange data only inside the warp and
-  // synchronise with __syncwarp instead of a CTA barrier (2^24: the load and
-  // three of the four stage pairs of every pass). ----
-  constexpr uint32_t W = THREADS / 32;
-  static_assert(TILE_MAX / THREADS >= 4, "each warp stages whole 128-element slices");
-  const uint32_t lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-  for (uint32_t r = 0; r < 2 * TILE_MAX / THREADS; r++) {
-    const uint32_t u = lane + 32 * (r & 7);
-    const uint32_t e = (warp + (r >> 3) * W) * 128 + (u >> 1), h = u & 1;
-    if (FULL || e < tile) {
-      const uint32_t col = e & (C - 1), t = e >> c;
-      uint32_t g;
-      uint4 val;
-      if (first) {
-        g = (rev_bits(t, k) << xcols_log) + col0 + col;
-        if (EXT && g >= src_len) val = make_uint4(0, 0, 0, 0);
-        else val = load_data<COHERENT>(pp.src + ((g << 1) | h));
-      } else {
-        g = hi_base + (t << S) + m0 + col;
-        val = load_data<COHERENT>(pp.src + ((g << 1) | h));
-      }
-      sm[h * TILE_MAX + e] = val;
+  __device__ __forceinline__ TilePass(const PassParams& p, uint32_t b, uint4* s)
+      : pp(p), sm(s), k(p.k), c(p.c), C(1u << p.c), S(p.S), first(p.first), inverse(p.inverse),
+        unit0(p.inverse | p.tw0_one), wide(p.wide), tw(p.tw) {
+    if (first) {
+      col0 = b << c;
+    } else {
+      const uint32_t mlog = S - c;
+      hi_base = (b >> mlog) << (S + k);
+      m0 = (b & ((1u << mlog) - 1)) << c;
     }
   }
-  // A radix-4 pair whose h satisfies (h << (c + 2)) <= 128 is warp-local.
-  if (k >= 2 && (C << 2) <= 128u) __syncwarp();
-  else __syncthreads();
 
-  // ---- radix-4 groups: stages i and i+1 on four elements in registers ----
-  uint32_t i = 1;
-  for (; i < k; i += 2) {
-    const uint32_t h = 1u << (i - 1);
+  // Element (row t, column col) of the input (`rev`: t bit-reversed in k bits,
+  // the natural-order row the first pass gathers) and of the output.
+  __device__ __forceinline__ fe load(uint32_t t, uint32_t rev, uint32_t col) const {
+    uint32_t g;
+    if (first) {
+      g = (rev << (pp.log_n - k)) + col0 + col;
+      if (EXT && g >= pp.src_len) {
+        fe z;
+#pragma unroll
+        for (int q = 0; q < 8; q++) z.v[q] = 0;
+        return z;
+      }
+    } else {
+      g = hi_base + (t << S) + m0 + col;
+    }
+    return load_data<COHERENT>(pp.src + ((uint64_t)g << 1), wide);
+  }
+  __device__ __forceinline__ uint32_t out_base(uint32_t col) const {
+    return first ? rev_bits(col0 + col, pp.log_n - k) << k : hi_base + m0 + col;
+  }
+  __device__ __forceinline__ void store(uint32_t base, uint32_t t, const fe& x, bool last) const {
+    const uint32_t g = base + (t << S);  // S == 0 in the first pass
+    fe y = x;
+    if (SCALE && pp.scale) {
+      const uint4* f = pp.scale_tab;
+      if (EXT && pp.scale != kScaleFixed) f += (pp.scale == kScaleElements ? 2ull : 4ull) * g;
+      if (EXT && pp.scale == kScaleElements) y = fe_mul<F>(fe_load_nc(f), x);
+      else y = fe_reduce<F>(fe_mul_fixed<F>(x, ld_fe32(f), ld_fe32(f + 2)));
+    } else if (last) {
+      y = fe_canonical<F>(x);
+    }
+    if (!EXT || g < pp.dst_len) store_data(pp.dst + ((uint64_t)g << 1), y, wide);
+  }
+
+  // Stages i and i+1 on four elements in registers (rows t0 + {0, h, 2h, 3h}).
+  // With u, v -> u + t, u - t, t = tw[j] v, the inverse (inttWithTwiddles: factor
+  // one for j = 0, else -tw[2^(s-1) - j]) is the same butterfly with the two
+  // results exchanged, so it reads the mirrored entry and exchanges where they
+  // go: the first stage's through the choice of the second stage's factors,
+  // the second's through the rows.
+  template <bool IN, bool OUT>
+  __device__ __forceinline__ void pair(uint32_t i, uint32_t ga, bool last) const {
+    const uint32_t h = IN ? 1u : 1u << (i - 1);
     const uint32_t half1 = 1u << (S + i - 1);  // stage S+i
     const uint32_t half2 = half1 << 1;         // stage S+i+1
-    const uint4* stw1 = tw + ((half1 - 1) << 1);
-    const uint4* stw2 = tw + ((half2 - 1) << 1);
+    const uint4* stw1 = tw + 4ull * (half1 - 1);
+    const uint4* stw2 = tw + 4ull * (half2 - 1);
+    const uint32_t col = ga & (C - 1), g = ga >> c;
+    const uint32_t j = g & (h - 1);
+    const uint32_t t0 = IN ? g << 2 : ((g >> (i - 1)) << (i + 1)) | j;
+    const uint32_t e0 = (t0 << c) | col, eh = h << c;
+    uint32_t jg1, jg3;
+    if (first) {
+      jg1 = j;
+      jg3 = j + h;
+    } else {
+      jg1 = (j << S) + m0 + col;
+      jg3 = jg1 + (h << S);
+    }
+    const bool mul = !(jg1 == 0 && unit0);
+    const bool swap = inverse && jg1 != 0;  // first-stage results exchanged
+    const uint32_t i1 = inverse ? half1 - jg1 : jg1;
+    // Second stage: the sums' pair and the differences' pair.
+    const uint32_t jp = swap ? jg3 : jg1, jm = swap ? jg1 : jg3;
+    const uint32_t ip = inverse ? half2 - jp : jp, im = inverse ? half2 - jm : jm;
+    fe x0, x1, x2, x3;
+    if constexpr (IN) {
+      const uint32_t rv = first ? rev_bits(t0, k) : 0;  // t0 is a multiple of 4
+      x1 = load(t0 + 1, rv + (1u << (k - 1)), col);
+      x0 = load(t0, rv, col);
+      x3 = load(t0 + 3, rv + (3u << (k - 2)), col);
+      x2 = load(t0 + 2, rv + (1u << (k - 2)), col);
+    }
+    fe p0, d0, p2, d2, y, z;
+    {
+      if constexpr (!IN) x1 = sm_load<TILE_MAX>(sm, e0 + eh);
+      const fe t = times_factor<F>(mul, stw1, i1, x1);
+      if constexpr (!IN) x0 = sm_load<TILE_MAX>(sm, e0);
+      fe_butterfly<F>(fe_weak<F>(x0), t, p0, d0);
+    }
+    {
+      if constexpr (!IN) x3 = sm_load<TILE_MAX>(sm, e0 + 3 * eh);
+      const fe t = times_factor<F>(mul, stw1, i1, x3);
+      if constexpr (!IN) x2 = sm_load<TILE_MAX>(sm, e0 + 2 * eh);
+      fe_butterfly<F>(fe_weak<F>(x2), t, p2, d2);
+    }
+    const uint32_t base = OUT ? out_base(col) : 0;
+    {
+      const fe t = times_factor<F>(mul, stw2, ip, p2);
+      if constexpr (!F::kLazy) p0 = fe_weak<F>(p0);
+      fe_butterfly<F>(p0, t, y, z);
+      const uint32_t a = swap ? 3 : 0, b = swap ? 1 : 2;  // rows of the sum and of the difference
+      if constexpr (OUT) {
+        store(base, t0 + a * h, y, last);
+        store(base, t0 + b * h, z, last);
+      } else {
+        sm_store<TILE_MAX>(sm, e0 + a * eh, y);
+        sm_store<TILE_MAX>(sm, e0 + b * eh, z);
+      }
+    }
+    {
+      const fe t = times_factor<F>(true, stw2, im, d2);
+      if constexpr (!F::kLazy) d0 = fe_weak<F>(d0);
+      fe_butterfly<F>(d0, t, y, z);
+      const uint32_t a0 = swap ? 0 : 1;
+      const uint32_t a = inverse ? a0 + 2 : a0, b = inverse ? a0 : a0 + 2;
+      if constexpr (OUT) {
+        store(base, t0 + a * h, y, last);
+        store(base, t0 + b * h, z, last);
+      } else {
+        sm_store<TILE_MAX>(sm, e0 + a * eh, y);
+        sm_store<TILE_MAX>(sm, e0 + b * eh, z);
+      }
+    }
+  }
+
+  // Stage k alone, at the end of a pass of odd k: rows t0 and t0 + 2^(k-1).
+  template <bool IN>
+  __device__ __forceinline__ void single(uint32_t ga, bool last) const {
+    const uint32_t h = 1u << (k - 1);
+    const uint32_t half = 1u << (S + k - 1);  // stage S+k
+    const uint4* stw = tw + 4ull * (half - 1);
+    const uint32_t col = ga & (C - 1), j = ga >> c;
+    const uint32_t jg = first ? j : (j << S) + m0 + col;
+    const bool swap = inverse && jg != 0;
+    const uint32_t e0 = (j << c) | col;
+    fe u, v, y, z;
+    if constexpr (IN) {
+      v = load(1, 1, col);
+      u = load(0, 0, col);
+    } else {
+      v = sm_load<TILE_MAX>(sm, e0 + (h << c));
+    }
+    const fe t = times_factor<F>(!(jg == 0 && unit0), stw, inverse ? half - jg : jg, v);
+    if constexpr (!IN) u = sm_load<TILE_MAX>(sm, e0);
+    fe_butterfly<F>(fe_weak<F>(u), t, y, z);
+    const uint32_t base = out_base(col);
+    store(base, swap ? j + h : j, y, last);
+    store(base, swap ? j : j + h, z, last);
+  }
+
+  __device__ __forceinline__ void run() const {
+    const uint32_t tile = FULL ? TILE_MAX : 1u << (k + c);
+    const uint32_t tid = threadIdx.x;
+    const bool last = S + k == pp.log_n;  // the transform's last stages: canonical results
+    if (k <= 2) {
+      // One group, straight from input to output (k == 0: a length-1 vector).
+      if (k == 2) {
+        for (uint32_t ga = tid; ga < tile / 4; ga += THREADS) pair<true, true>(1, ga, last);
+      } else if (k == 1) {
+        for (uint32_t ga = tid; ga < tile / 2; ga += THREADS) single<true>(ga, last);
+      } else if (tid == 0) {
+        store(0, 0, load(0, 0, 0), false);
+      }
+      return;
+    }
+    // Warp w's groups of a pair of span 4 h C <= 128 elements are the same
+    // 128-element slices of the tile: such pairs exchange data only inside the
+    // warp and synchronise with __syncwarp, the others with a CTA barrier
+    // (2^24: two of the three exchanges of every pass are warp-local).
 #pragma unroll
     for (uint32_t q = 0; q < TILE_MAX / 4 / THREADS; q++) {
       const uint32_t ga = tid + q * THREADS;
-      if (FULL || ga < tile / 4) {
-        const uint32_t col = ga & (C - 1), g = ga >> c;
-        const uint32_t j = g & (h - 1);
-        const uint32_t t0 = ((g >> (i - 1)) << (i + 1)) | j;
-        const uint32_t e0 = (t0 << c) | col, eh = h << c;
-        uint32_t jg1, jg3;
-        if (first) {
-          jg1 = j;
-          jg3 = j + h;
-        } else {
-          jg1 = (j << S) + m0 + col;
-          jg3 = jg1 + (h << S);
-        }
-        fe w1, w2, w3;
-        const bool m1 = twiddle<F>(inverse, unit0, stw1, half1, jg1, w1);
-        const bool m2 = twiddle<F>(inverse, unit0, stw2, half2, jg1, w2);
-        const bool m3 = twiddle<F>(inverse, unit0, stw2, half2, jg3, w3);
-        fe x0 = sm_load<TILE_MAX>(sm, e0), x1 = sm_load<TILE_MAX>(sm, e0 + eh),
-           x2 = sm_load<TILE_MAX>(sm, e0 + 2 * eh), x3 = sm_load<TILE_MAX>(sm, e0 + 3 * eh);
-        butterfly<F>(x0, x1, m1, w1);
-        butterfly<F>(x2, x3, m1, w1);
-        butterfly<F>(x0, x2, m2, w2);
-        butterfly<F>(x1, x3, m3, w3);
-        const bool last = i + 2 > k;
-        canonical<F>(x0, last);
-        canonical<F>(x1, last);
-        canonical<F>(x2, last);
-        canonical<F>(x3, last);
-        sm_store<TILE_MAX>(sm, e0, x0);
-        sm_store<TILE_MAX>(sm, e0 + eh, x1);
-        sm_store<TILE_MAX>(sm, e0 + 2 * eh, x2);
-        sm_store<TILE_MAX>(sm, e0 + 3 * eh, x3);
+      if (FULL || ga < tile / 4) pair<true, false>(1, ga, false);
+    }
+    uint32_t i = 3;
+    for (;; i += 2) {
+      // Stages i, i+1 next: their span is 2^(i+1) C.
+      if (((2u << i) << c) <= 128u) __syncwarp();
+      else __syncthreads();
+      if (i + 1 >= k) break;
+#pragma unroll
+      for (uint32_t q = 0; q < TILE_MAX / 4 / THREADS; q++) {
+        const uint32_t ga = tid + q * THREADS;
+        if (FULL || ga < tile / 4) pair<false, false>(i, ga, false);
       }
     }
-    // The next pair (stages i+2, i+3) is warp-local when its h = 2^(i+1) is.
-    if (i + 2 < k && ((2u << i) << (c + 2)) <= 128u) __syncwarp();
-    else __syncthreads();
+    if (i + 1 == k) {
+#pragma unroll
+      for (uint32_t q = 0; q < TILE_MAX / 4 / THREADS; q++) {
+        const uint32_t ga = tid + q * THREADS;
+        if (FULL || ga < tile / 4) pair<false, true>(i, ga, last);
+      }
+    } else {
+      // An odd stage count ends with one radix-2 stage.  Last rather than
+      // first: in a transform's first pass the first stage pair then holds the
+      // factors that are one (stage 1, and stage 2's j = 0), so the pass skips
+      // their products in whole warps (2^20 first pass 8% faster, B200).
+#pragma unroll
+      for (uint32_t q = 0; q < TILE_MAX / 2 / THREADS; q++) {
+        const uint32_t ga = tid + q * THREADS;
+        if (FULL || ga < tile / 2) single<false>(ga, last);
+      }
+    }
   }
+};
 
-  // ---- an odd stage count ends with one radix-2 stage (stage k of the pass).
-  // Last rather than first: in a transform's first pass the first stage pair
-  // then holds the factors that are one (stage 1, and stage 2's j = 0), so the
-  // pass skips their products in whole warps (2^20 first pass 8% faster, B200).
-  if (k & 1) {
-    const uint32_t h = 1u << (k - 1);
-    const uint32_t half_g = 1u << (S + k - 1);  // stage S+k
-    const uint4* stw = tw + ((half_g - 1) << 1);
-#pragma unroll
-    for (uint32_t q = 0; q < TILE_MAX / 2 / THREADS; q++) {
-      const uint32_t b = tid + q * THREADS;
-      if (FULL || b < tile / 2) {
-        const uint32_t col = b & (C - 1), g = b >> c;
-        const uint32_t j = g & (h - 1);
-        const uint32_t t0 = ((g >> (k - 1)) << k) | j;
-        const uint32_t jg = first ? j : (j << S) + m0 + col;
-        const uint32_t e0 = (t0 << c) | col, e1 = e0 + (h << c);
-        fe u = sm_load<TILE_MAX>(sm, e0), v = sm_load<TILE_MAX>(sm, e1), w;
-        const bool mul = twiddle<F>(inverse, unit0, stw, half_g, jg, w);
-        butterfly<F>(u, v, mul, w);
-        canonical<F>(u, true);
-        canonical<F>(v, true);
-        sm_store<TILE_MAX>(sm, e0, u);
-        sm_store<TILE_MAX>(sm, e1, v);
-      }
-    }
-    __syncthreads();
-  }
-
-  // ---- the inverse's 1/n (or a per-position factor table), then store ----
-  if (SCALE && pp.scale) {
-    fe sc;
-#pragma unroll
-    for (int q = 0; q < 8; q++) sc.v[q] = pp.scale_val[q];
-#pragma unroll
-    for (uint32_t q = 0; q < TILE_MAX / THREADS; q++) {
-      const uint32_t e = tid + q * THREADS;
-      if (FULL || e < tile) {
-        const uint32_t col = e & (C - 1), row = e >> c;
-        if (EXT && pp.scale_tab) {
-          const uint32_t g = first ? (rev_bits(col0 + col, xcols_log) << k) + row : hi_base + (row << S) + m0 + col;
-          sc = fe_load_nc(pp.scale_tab + (g << 1));
-        }
-        sm_store<TILE_MAX>(sm, e, fe_mul<F>(sm_load<TILE_MAX>(sm, e), sc));
-      }
-    }
-    __syncthreads();
-  }
-
-#pragma unroll
-  for (uint32_t q = 0; q < 2 * TILE_MAX / THREADS; q++) {
-    const uint32_t idx = tid + q * THREADS;
-    if (FULL || idx < 2 * tile) {
-      const uint32_t h = idx & 1, e = idx >> 1, col = e & (C - 1), row = e >> c;
-      uint32_t g;
-      if (first) {
-        g = (rev_bits(col0 + col, xcols_log) << k) + row;
-      } else {
-        g = hi_base + (row << S) + m0 + col;
-      }
-      if (!EXT || g < pp.dst_len) pp.dst[(g << 1) | h] = sm[h * TILE_MAX + ((row << c) | col)];
-    }
-  }
+template <class F, int LOG_TILE, int THREADS, bool COHERENT, bool EXT, bool FULL = false, bool SCALE = true>
+__device__ __forceinline__ void ntt_tile(const PassParams& pp, uint32_t blk, uint4* sm) {
+  TilePass<F, LOG_TILE, THREADS, COHERENT, EXT, FULL, SCALE>(pp, blk, sm).run();
 }
 
 }  // namespace zntt

@@ -159,7 +159,10 @@ struct PoolBuf {
 // Up to log_tile stages run in one pass on a single tile of 2^log_n <=
 // 2^log_tile elements.  Longer transforms are split into P = ceil(log_n / kmax)
 // passes of near-equal stage counts; each tile keeps 2^log_tile elements, the
-// spare bits becoming 2^c contiguous positions per tile row.
+// spare bits becoming 2^c contiguous positions per tile row.  (Dealing the
+// stages out in pairs, 2^22 as 8 + 8 + 6 rather than 8 + 7 + 7, saves the odd
+// passes' radix-2 exchange but narrows rows: 2^22 BLS12-381-Fr 0.688 -> 0.694 ms,
+// 64 extensions 2^18 -> 2^20 11.75 -> 11.98 ms, B200; not used.)
 Plan make_plan(uint32_t log_n, int shape, uint32_t kmax) {
   Plan plan;
   plan.shape = shape;
@@ -199,7 +202,7 @@ Plan tuned_plan(int field, uint32_t log_n) {
 }
 
 int run_plan(int field, const TwEntry* tw, const Plan& plan, uint32_t log_n, const uint4* d_src, uint4* d_dst,
-             uint4* d_scratch, bool inverse, bool scale, const uint64_t* scale_val, cudaStream_t st) {
+             uint4* d_scratch, bool inverse, bool scale, cudaStream_t st) {
   if (log_n == 0) {
     // A length-1 transform has no stages; the inverse scale is by 1/1 = 1.
     if (d_src != d_dst) ZCHECK(cudaMemcpyAsync(d_dst, d_src, 32, cudaMemcpyDeviceToDevice, st), "copy");
@@ -216,6 +219,7 @@ int run_plan(int field, const TwEntry* tw, const Plan& plan, uint32_t log_n, con
     pp.src = cur_src;
     pp.dst = last ? d_dst : mid;
     pp.tw = tw->d_table;
+    pp.wide = pass_wide(pp.src, pp.dst);
     pp.log_n = log_n;
     pp.S = d.S;
     pp.k = d.k;
@@ -223,8 +227,8 @@ int run_plan(int field, const TwEntry* tw, const Plan& plan, uint32_t log_n, con
     pp.first = p == 0;
     pp.inverse = inverse;
     pp.tw0_one = tw->tw0_one;
-    pp.scale = last && scale;
-    if (pp.scale) std::memcpy(pp.scale_val, scale_val, 32);
+    pp.scale = last && scale ? kScaleFixed : kScaleNone;
+    pp.scale_tab = tw->n_inv();
     pp.src_len = 1ull << log_n;
     pp.dst_len = 1ull << log_n;
     const uint64_t tiles = (1ull << log_n) >> (d.k + d.c);
@@ -235,9 +239,8 @@ int run_plan(int field, const TwEntry* tw, const Plan& plan, uint32_t log_n, con
 }
 
 int run_transform(int field, const TwEntry* tw, uint32_t log_n, const uint4* d_src, uint4* d_dst, uint4* d_scratch,
-                  bool inverse, bool scale, const uint64_t* scale_val, cudaStream_t st) {
-  return run_plan(field, tw, tuned_plan(field, log_n), log_n, d_src, d_dst, d_scratch, inverse, scale, scale_val,
-                  st);
+                  bool inverse, bool scale, cudaStream_t st) {
+  return run_plan(field, tw, tuned_plan(field, log_n), log_n, d_src, d_dst, d_scratch, inverse, scale, st);
 }
 
 int pool_get(size_t bytes, void** out) {
@@ -262,11 +265,12 @@ static std::string table_key(int field, uint32_t log_n, const uint64_t* root) {
   return buf;
 }
 
-static size_t table_entries(uint32_t log_n) { return log_n == 0 ? 1 : ((size_t)1 << log_n) - 1; }
+static size_t table_bytes(uint32_t log_n) { return (size_t)64 << log_n; }
 
 static void free_entry(TwEntry* e) {
   Context& c = ctx();
   if (e->d_table) cudaFree(e->d_table);
+  if (e->upload) c.pool.release(e->upload, e->upload_bytes);
   c.all_tables.erase(std::remove(c.all_tables.begin(), c.all_tables.end(), e), c.all_tables.end());
   for (auto it = c.tw_by_key.begin(); it != c.tw_by_key.end(); ++it) {
     if (it->second == e) {
@@ -315,14 +319,15 @@ void host_power_tables(int field, const uint64_t* base, std::vector<uint64_t>& p
 }
 
 static int fill_table(TwEntry* e, cudaStream_t st) {
-  if (e->log_n == 0) return ZNTT_OK;
   std::vector<uint64_t> pw;
   host_power_tables(e->field, e->root, pw);
   PoolBuf d_pw;
   int rc = d_pw.get(pw.size() * 8);
   if (rc) return rc;
   ZCHECK(cudaMemcpyAsync(d_pw.p, pw.data(), pw.size() * 8, cudaMemcpyHostToDevice, st), "twiddle powers upload");
-  ZCHECK(launch_twiddle_table(e->field, (const uint4*)d_pw.p, e->d_table, e->log_n, st), "twiddle kernel");
+  uint64_t ninv[4];
+  n_inverse(e->field, e->log_n, ninv);
+  ZCHECK(launch_twiddle_table(e->field, (const uint4*)d_pw.p, ninv, e->d_table, e->log_n, st), "twiddle kernel");
   ZCHECK(cudaStreamSynchronize(st), "twiddle kernel");
   return ZNTT_OK;
 }
@@ -342,7 +347,7 @@ int acquire_table(int field, uint32_t log_n, const uint64_t* root, TwEntry** out
   e->field = field;
   e->log_n = log_n;
   std::memcpy(e->root, root, 32);
-  e->bytes = table_entries(log_n) * 32;
+  e->bytes = table_bytes(log_n);
   evict_tables(e->bytes);
   cudaError_t ce = cudaMalloc((void**)&e->d_table, e->bytes);
   if (ce == cudaErrorMemoryAllocation) {
@@ -389,22 +394,35 @@ static int upload_foreign_table(int field, uint32_t log_n, const zntt_stage* sta
   e->field = field;
   e->log_n = log_n;
   e->foreign = true;
-  e->bytes = table_entries(log_n) * 32;
+  e->bytes = table_bytes(log_n);
   cudaError_t ce = cudaMalloc((void**)&e->d_table, e->bytes);
   if (ce != cudaSuccess) {
     delete e;
     return cuda_fail(ce, "foreign twiddle table");
   }
+  e->upload_bytes = (size_t)32 << log_n;
+  int rc = pool_get(e->upload_bytes, &e->upload);
+  if (rc) {
+    cudaFree(e->d_table);
+    delete e;
+    return rc;
+  }
   e->tw0_one = true;
   for (uint32_t s = 0; s < log_n; s++) {
     if (!F.is_one(stages[s].ptr)) e->tw0_one = false;
-    ce = cudaMemcpyAsync(e->d_table + 2 * (((size_t)1 << s) - 1), stages[s].ptr, ((size_t)1 << s) * 32,
-                         cudaMemcpyHostToDevice, c.stream);
-    if (ce != cudaSuccess) {
-      cudaFree(e->d_table);
-      delete e;
-      return cuda_fail(ce, "foreign twiddle upload");
-    }
+    if (ce == cudaSuccess)
+      ce = cudaMemcpyAsync((uint4*)e->upload + 2 * (((size_t)1 << s) - 1), stages[s].ptr, ((size_t)1 << s) * 32,
+                           cudaMemcpyHostToDevice, c.stream);
+  }
+  uint64_t ninv[4];
+  n_inverse(field, log_n, ninv);
+  if (ce == cudaSuccess) ce = launch_twiddle_pairs(field, (const uint4*)e->upload, ninv, e->d_table, log_n, c.stream);
+  if (ce != cudaSuccess) {
+    cudaStreamSynchronize(c.stream);
+    cudaFree(e->d_table);
+    pool_put(e->upload, e->upload_bytes);
+    delete e;
+    return cuda_fail(ce, "foreign twiddle upload");
   }
   e->refs = 1;
   c.all_tables.push_back(e);
@@ -432,8 +450,7 @@ static Registration* find_registration(int field, uint32_t log_n, const zntt_sta
 // host-data transform
 // ---------------------------------------------------------------------------
 
-static int transform_host(int field, uint64_t* data, uint32_t log_n, const TwEntry* tw, bool inverse, bool scale,
-                          const uint64_t* scale_val) {
+static int transform_host(int field, uint64_t* data, uint32_t log_n, const TwEntry* tw, bool inverse, bool scale) {
   Context& c = ctx();
   const size_t n = (size_t)1 << log_n;
   const size_t bytes = n * 32;
@@ -443,7 +460,7 @@ static int transform_host(int field, uint64_t* data, uint32_t log_n, const TwEnt
   rc = b.get(bytes);
   if (rc) return rc;
   ZCHECK(cudaMemcpyAsync(a.p, data, bytes, cudaMemcpyHostToDevice, c.stream), "upload");
-  rc = run_transform(field, tw, log_n, (const uint4*)a.p, (uint4*)b.p, nullptr, inverse, scale, scale_val, c.stream);
+  rc = run_transform(field, tw, log_n, (const uint4*)a.p, (uint4*)b.p, nullptr, inverse, scale, c.stream);
   if (rc) return rc;
   ZCHECK(cudaMemcpyAsync(data, b.p, bytes, cudaMemcpyDeviceToHost, c.stream), "download");
   ZCHECK(cudaStreamSynchronize(c.stream), "transform");
@@ -513,9 +530,7 @@ static int ntt_with_twiddles_impl(int field, uint64_t* data, size_t len, size_t 
     if (rc) return rc;
     foreign = true;
   }
-  uint64_t ninv[4];
-  if (inverse) n_inverse(field, (uint32_t)log_n, ninv);
-  rc = transform_host(field, data, (uint32_t)log_n, tw, inverse, inverse, ninv);
+  rc = transform_host(field, data, (uint32_t)log_n, tw, inverse, inverse);
   if (foreign) {
     cudaStreamSynchronize(c.stream);
     release_table(tw);
@@ -546,9 +561,7 @@ static int ntt_root_impl(int field, uint64_t* data, size_t len, size_t log_n, co
   TwEntry* tw = nullptr;
   rc = acquire_table(field, (uint32_t)log_n, r, &tw);
   if (rc) return rc;
-  uint64_t ninv[4];
-  if (inverse) n_inverse(field, (uint32_t)log_n, ninv);
-  rc = transform_host(field, data, (uint32_t)log_n, tw, false, inverse, ninv);
+  rc = transform_host(field, data, (uint32_t)log_n, tw, false, inverse);
   release_table(tw);
   return rc;
 }
@@ -729,15 +742,27 @@ int zntt_precompute_twiddles(int field, size_t log_n, const uint64_t root[4], ui
   TwEntry* tw = nullptr;
   rc = acquire_table(field, (uint32_t)log_n, root, &tw);
   if (rc) return rc;
+  // The caller's table holds the entries in Montgomery form: made from the
+  // device's fixed factors in pieces of at most 2^22 entries.
+  const size_t piece = std::min<size_t>((size_t)1 << 22, (size_t)1 << (log_n - 1));
+  PoolBuf d_entries;
+  rc = d_entries.get(piece * 32);
+  if (rc) {
+    release_table(tw);
+    return rc;
+  }
+  cudaError_t e = cudaSuccess;
   for (size_t s = 0; s < log_n; s++) {
-    cudaError_t e = cudaMemcpyAsync(stage_out[s], tw->d_table + 2 * (((size_t)1 << s) - 1), ((size_t)1 << s) * 32,
-                                    cudaMemcpyDeviceToHost, c.stream);
-    if (e != cudaSuccess) {
-      release_table(tw);
-      return cuda_fail(e, "twiddle download");
+    const size_t len = (size_t)1 << s;
+    for (size_t at = 0; at < len && e == cudaSuccess; at += piece) {
+      const size_t m = std::min(piece, len - at);
+      e = launch_pair_entries(field, tw->d_table + 4 * (len - 1 + at), (uint4*)d_entries.p, m, c.stream);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(stage_out[s] + 4 * at, d_entries.p, m * 32, cudaMemcpyDeviceToHost, c.stream);
     }
   }
-  cudaError_t e = cudaStreamSynchronize(c.stream);
+  const cudaError_t se = cudaStreamSynchronize(c.stream);
+  if (e == cudaSuccess) e = se;
   if (e != cudaSuccess) {
     release_table(tw);
     return cuda_fail(e, "twiddle download");
@@ -861,8 +886,6 @@ int zntt_ntt_device(const zntt_twiddles* tw, const uint64_t* d_src, uint64_t* d_
   const TwEntry* e = reinterpret_cast<const TwEntry*>(tw);
   cudaStream_t st = stream ? (cudaStream_t)stream : c.stream;
   const bool inverse = mode == ZNTT_INVERSE;
-  uint64_t ninv[4];
-  if (inverse) n_inverse(e->field, e->log_n, ninv);
   const bool need_scratch = d_src == d_dst && tuned_plan(e->field, e->log_n).np > 1;
   if (need_scratch && !d_scratch) {
     // Borrow a pool buffer; it returns to the pool only after the stream has
@@ -871,14 +894,14 @@ int zntt_ntt_device(const zntt_twiddles* tw, const uint64_t* d_src, uint64_t* d_
     rc = s.get(((size_t)1 << e->log_n) * 32);
     if (rc) return rc;
     rc = run_transform(e->field, e, e->log_n, (const uint4*)d_src, (uint4*)d_dst, (uint4*)s.p, inverse, inverse,
-                       ninv, st);
+                       st);
     cudaError_t ce = cudaStreamSynchronize(st);
     if (rc) return rc;
     if (ce != cudaSuccess) return cuda_fail(ce, "transform");
     return ZNTT_OK;
   }
   return run_transform(e->field, e, e->log_n, (const uint4*)d_src, (uint4*)d_dst, (uint4*)d_scratch, inverse,
-                       inverse, ninv, st);
+                       inverse, st);
 }
 
 int zntt_elementwise_device(int field, int op, const uint64_t* d_a, const uint64_t* d_b, uint64_t* d_out,

@@ -15,17 +15,21 @@
 
 namespace zntt {
 
-// A device twiddle table in zig-ntt's flat layout (stage s at entry 2^s - 1).
+// A device twiddle table in zig-ntt's flat layout (stage s at entry 2^s - 1), as
+// fixed factors of 64 bytes (shoup.cuh), and 1/n as its last entry.
 struct TwEntry {
   int field = 0;
   uint32_t log_n = 0;
   uint64_t root[4] = {0, 0, 0, 0};  // Montgomery form; the key of root-derived tables
-  uint4* d_table = nullptr;         // 2^log_n - 1 entries (one entry when log_n == 0)
+  uint4* d_table = nullptr;         // 2^log_n entries of 4 uint4
   size_t bytes = 0;
   int refs = 0;                     // handles + registrations holding it
   bool tw0_one = true;              // every stage's entry 0 equals one
   bool foreign = false;             // uploaded from a caller's table, not derived from a root
   uint64_t last_use = 0;
+  void* upload = nullptr;           // a foreign table's entries as given (pool buffer, released with the table)
+  size_t upload_bytes = 0;
+  const uint4* n_inv() const { return d_table + 4 * (((size_t)1 << log_n) - 1); }
 };
 
 // A host table made by zntt_precompute_twiddles, recognised again by its stage
@@ -120,12 +124,12 @@ void release_table(TwEntry* e);
 // Runs the DIT network over 2^log_n device elements: d_src -> d_dst, with
 // d_scratch (2^log_n elements) used when d_src == d_dst and there are several
 // passes.  `inverse` selects the inttWithTwiddles twiddle mapping; `scale`
-// multiplies every output by `scale_val` (Montgomery form) after the last stage.
+// multiplies every output by 1/n after the last stage.
 int run_transform(int field, const TwEntry* tw, uint32_t log_n, const uint4* d_src, uint4* d_dst,
-                  uint4* d_scratch, bool inverse, bool scale, const uint64_t* scale_val, cudaStream_t st);
+                  uint4* d_scratch, bool inverse, bool scale, cudaStream_t st);
 // The same with an explicit plan (used by the autotuner).
 int run_plan(int field, const TwEntry* tw, const Plan& plan, uint32_t log_n, const uint4* d_src, uint4* d_dst,
-             uint4* d_scratch, bool inverse, bool scale, const uint64_t* scale_val, cudaStream_t st);
+             uint4* d_scratch, bool inverse, bool scale, cudaStream_t st);
 
 // Pool buffer helpers shared by the translation units.
 int pool_get(size_t bytes, void** out);

@@ -296,11 +296,9 @@ static bool launch_into(zntt_server* s, Slot& sl) {
     }
     if (r.kind == ZNTT_JOB_NTT) {
       const bool inv = r.mode == ZNTT_INVERSE;
-      uint64_t ninv[4];
-      if (inv) n_inverse(field, r.log_n, ninv);
       const Plan plan = batch_plan(field, r.log_n, shape);
       plan_transform(plans[j], tw, plan, r.log_n, (const uint4*)q.d_in, (uint4*)q.d_out, (uint4*)q.d_out, inv,
-                     inv ? ninv : nullptr, nullptr, 1ull << r.log_n, 1ull << r.log_n);
+                     inv ? kScaleFixed : kScaleNone, tw->n_inv(), 1ull << r.log_n, 1ull << r.log_n);
     } else {
       TwEntry* twi = nullptr;
       rc = table_for(s, r.log_in, &twi);
@@ -312,9 +310,9 @@ static bool launch_into(zntt_server* s, Slot& sl) {
       const Plan pi = batch_plan(field, r.log_in, shape);
       const Plan po = batch_plan(field, r.log_n, shape);
       plan_transform(plans[j], twi, pi, r.log_in, (const uint4*)q.d_in, (uint4*)q.d_coef, (uint4*)q.d_coef, true,
-                     nullptr, q.ct->d, 1ull << r.log_in, 1ull << r.log_in);
+                     kScaleFixedTab, q.ct->d, 1ull << r.log_in, 1ull << r.log_in);
       plan_transform(plans[j], tw, po, r.log_n, (const uint4*)q.d_coef, (uint4*)q.d_out, (uint4*)q.d_out, false,
-                     nullptr, nullptr, 1ull << r.log_in, 1ull << r.log_n);
+                     kScaleNone, nullptr, 1ull << r.log_in, 1ull << r.log_n);
     }
   }
 
