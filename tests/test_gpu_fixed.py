@@ -90,3 +90,33 @@ def test_extension_between_misaligned_vectors(z):
             torch.cuda.synchronize()
             b.status()
         assert np.array_equal(dst[2:].cpu().numpy().view(np.uint64).reshape(-1, 4), want.reshape(-1, 4))
+
+
+@pytest.mark.parametrize("log_n", [1, 7, 8, 9, 15, 16, 17, 20])
+def test_captured_transforms_replay(z, log_n):
+    """Transforms captured by the caller's CUDA graph (their passes' launches overlap) replay on
+    new data with the results of direct calls."""
+    import torch
+    F, n = z.BN254_FR, 1 << log_n
+    stream = torch.cuda.Stream()
+    with z.DeviceTwiddles(F, log_n, z.primitiveRootOfUnity(F, log_n)) as tw, torch.cuda.stream(stream):
+        src, mid, dst = (torch.zeros(4 * n, dtype=torch.int64, device="cuda") for _ in range(3))
+
+        def both():
+            z.ntt_device(tw, src.data_ptr(), mid.data_ptr(), z.FORWARD, stream=stream.cuda_stream)
+            z.ntt_device(tw, mid.data_ptr(), dst.data_ptr(), z.INVERSE, stream=stream.cuda_stream)
+
+        both()
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            both()
+        for seed in (1, 2):
+            z.random_elements(F, seed, src.data_ptr(), n, stream=stream.cuda_stream)
+            both()
+            want = mid.clone()
+            mid.zero_()
+            dst.zero_()
+            graph.replay()
+            stream.synchronize()
+            assert torch.equal(mid, want) and torch.equal(dst, src)

@@ -59,7 +59,16 @@ struct PassShape {
 // The last shape trades a 72-register budget (a few spilled words) for 28
 // warps per SM: 2^22 and 2^24 BN254-Fr about 0.6% faster, BLS12-381-Fr slower.
 constexpr int kNumShapes = 5;
-constexpr PassShape kShapes[kNumShapes] = {{11, 256, 3}, {10, 256, 3}, {9, 128, 6}, {8, 64, 12}, {9, 128, 7}};
+// Behind the tunable shapes, two of one butterfly per thread (ntt_tile_radix2),
+// kRadix2Shape with 2^7-element tiles and the next with 2^8.
+constexpr PassShape kShapes[kNumShapes + 2] = {{11, 256, 3}, {10, 256, 3}, {9, 128, 6}, {8, 64, 12},
+                                               {9, 128, 7},  {7, 64, 8},   {8, 128, 4}};
+constexpr int kRadix2Shape = kNumShapes;
+// Plain transforms up to this size run on the radix-2 shapes.  Both ways, two
+// transforms (forward and inverse) of BN254-Fr in us, B200: 2^10 24.6 against 37.1
+// with the tuned radix-4 passes, 2^14 31.7 / 47.1, 2^16 43.0 / 51.2, and from 2^17
+// on the radix-4 passes are as fast or faster (63.5 / 63.6, 2^18 106 / 102).
+constexpr uint32_t kRadix2MaxLog = 16;
 // The shape of persistent launches (batches and the server's slices): the
 // 7-CTA 2^9 tile ran the mixed 520-transform batch 3.03 -> 2.94 ms and 64
 // coset extensions 2^18 -> 2^20 16.95 -> 16.74 ms (BLS12-381-Fr) and 15.81 ->

@@ -85,9 +85,9 @@ extern "C" int zntt_ntt_device_inplace_noalloc(const zntt_twiddles* tw, uint64_t
     scratch = static_cast<uint4*>(g_noalloc_scratch_addr[dev]);
   }
 
-  // The library's planner (a plan is a value; planning allocates nothing): with 2^11-element
-  // tiles and at most 2^18 elements it gives one pass (log_n <= 11) or two.
-  const Plan plan = make_plan(log_n, kDefaultShape, kShapes[kDefaultShape].log_tile - 1);
+  // The library's planner (a plan is a value; planning allocates nothing): one pass or two.
+  const Plan plan = log_n <= kRadix2MaxLog ? radix2_plan(log_n)
+                                           : make_plan(log_n, kDefaultShape, kShapes[kDefaultShape].log_tile - 1);
   const uint32_t np = plan.np;
   const PassDesc* passes = plan.p;
 
@@ -116,7 +116,7 @@ extern "C" int zntt_ntt_device_inplace_noalloc(const zntt_twiddles* tw, uint64_t
     pp.src_len = 1ull << log_n;
     pp.dst_len = 1ull << log_n;
     const uint64_t tiles = (1ull << log_n) >> (pp.k + pp.c);
-    ce = launch_ntt_pass(e->field, kDefaultShape, pp, tiles, st);
+    ce = launch_ntt_pass(e->field, plan.shape, pp, tiles, st);
     if (ce != cudaSuccess) return cuda_fail(ce, "ntt pass launch");
   }
   return ZNTT_OK;

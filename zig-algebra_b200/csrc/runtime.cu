@@ -193,7 +193,14 @@ uint32_t tuned_kmax(int field, uint32_t log_n, int shape) {
   return kShapes[shape].log_tile - 1;
 }
 
+// One pass up to 2^8 elements, else two of half the stages each.
+Plan radix2_plan(uint32_t log_n) {
+  const uint32_t k = log_n <= 8 ? log_n : (log_n + 1) / 2;
+  return make_plan(log_n, k <= 7 ? kRadix2Shape : kRadix2Shape + 1, k);
+}
+
 Plan tuned_plan(int field, uint32_t log_n) {
+  if (log_n >= 1 && log_n <= kRadix2MaxLog) return radix2_plan(log_n);
   const TuneEntry* best = nullptr;
   for (const TuneEntry& t : ctx().tune)
     if (t.field == field && t.log_n == log_n && (!best || t.us < best->us)) best = &t;

@@ -53,8 +53,10 @@ struct Plan {
 };
 // Splits log_n stages into passes of at most kmax stages on tiles of the shape.
 Plan make_plan(uint32_t log_n, int shape, uint32_t kmax);
-// The plan the tuning table holds for (field, log_n), else the default shape
-// with kmax = log_tile - 1.
+// The plan on the radix-2 shapes for 1 <= log_n <= kRadix2MaxLog.
+Plan radix2_plan(uint32_t log_n);
+// The radix-2 plan for the sizes it serves, else the plan the tuning table holds
+// for (field, log_n), else the default shape with kmax = log_tile - 1.
 Plan tuned_plan(int field, uint32_t log_n);
 // The tuned stage count for a given shape.
 uint32_t tuned_kmax(int field, uint32_t log_n, int shape);
