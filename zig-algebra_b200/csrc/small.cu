@@ -5,9 +5,10 @@
 // An element is SmallField's canonical u64 (8 bytes).  The transform is the
 // same DIT network as the 256-bit path (root.zig:148-212; bit reversal folded
 // into the first pass, tiles of 2^k positions x 2^c neighbouring columns,
-// radix-4 register groups, 1/n fused into the last pass), on 8-byte elements
-// with tiles of 2^12 in shared memory.  Twiddle tables live on the device in
-// twiddle form (small_field.cuh); host tables handed across the C ABI are
+// 1/n fused into the last pass), on 8-byte elements with tiles of 2^12 in
+// shared memory: small_tile.cuh's passes on sixteen elements per thread, and
+// this file's on radix-4 groups for what those do not take.  Twiddle tables live
+// on the device as entries (small_field.cuh); host tables handed across the C ABI are
 // canonical, in zig-ntt's layout.
 #include <cuda_runtime.h>
 
@@ -20,6 +21,7 @@
 #include "runtime.hpp"
 #include "small.hpp"
 #include "small_field.cuh"
+#include "small_tile.cuh"
 
 namespace zntt {
 
@@ -57,27 +59,7 @@ const SmallHost& small_host(int field) { return field == kGoldilocksField ? kGol
 constexpr int kSmallLogTile = 12;
 constexpr int kSmallThreads = 256;
 constexpr uint32_t kSmallKmax = 10;  // keeps 2^(12 - k) >= 4 columns (32-byte rows) per tile row
-// Goldilocks transforms of 2^21 elements and more run on 2^11-element tiles in
-// CTAs of 128 threads (10 per SM): the same warps per SM in smaller CTAs, whose
-// barriers wait on fewer warps (2^24: 7.7% faster than 2^12 tiles in 256
-// threads, B200).  BabyBear gains nothing from it and keeps the larger tile.
-constexpr int kSmallLogTileB = 11;
-constexpr int kSmallThreadsB = 128;
-constexpr uint32_t kSmallKmaxB = 9;  // keeps 32-byte rows on 2^11-element tiles
-bool small_use_b(int field, uint32_t log_n) { return field == kGoldilocksField && log_n >= 21; }
-
-struct SmallPass {
-  const uint64_t* src;
-  uint64_t* dst;
-  const uint64_t* tw;  // twiddle form, stage s at entry 2^s - 1
-  uint32_t log_n, S, k, c, first, inverse, tw0_one, scale;
-  uint64_t scale_val;  // twiddle form
-  uint32_t src_len;    // column launches' first pass: natural index >= src_len reads as zero
-};
-
-__device__ __forceinline__ uint32_t rev_bits_small(uint32_t x, uint32_t bits) {
-  return bits == 0 ? 0u : (__brev(x) >> (32 - bits));
-}
+constexpr uint32_t kTileKmax = 10;   // the same on small_tile.cuh's tiles
 
 // Twiddle of global stage s for butterfly jg: forward tw[s-1][jg], inverse 1
 // (jg = 0) or -tw[s-1][2^(s-1) - jg] (root.zig:199); false when it is one.
@@ -86,26 +68,26 @@ template <class SF>
 __device__ __forceinline__ bool small_twiddle(const SmallPass& pp, const uint64_t* stw, uint32_t half, uint32_t jg,
                                               uint64_t& w) {
   if (jg == 0 && (pp.inverse | pp.tw0_one)) return false;
-  w = pp.inverse ? SF::neg(__ldg(stw + (half - jg))) : __ldg(stw + jg);
+  w = pp.inverse ? SF::neg_entry(__ldg(stw + (half - jg))) : __ldg(stw + jg);
   return true;
 }
 
 template <class SF>
 __device__ __forceinline__ void small_butterfly(uint64_t& u, uint64_t& v, bool mul, uint64_t w) {
-  const uint64_t t = mul ? SF::mul(w, v) : v;
+  const uint64_t t = mul ? SF::mul_entry(w, v) : v;
   v = SF::sub(u, t);
   u = SF::add(u, t);
 }
 
-// One tile of one pass.  PAD: the first pass reads natural indices at or
-// beyond pp.src_len as zeros (a zero-padded input that is not stored).  FULL:
-// the tile is the whole 2^LOG_TILE (k + c == LOG_TILE), so no bound checks
-// (2^24 BabyBear about 10% faster without them on B200).
-template <class SF, int LOG_TILE, int THREADS, bool PAD, bool FULL = false>
+// One tile of one pass, for what small_tile.cuh does not take: transforms below
+// 2^12 and caller tables whose entries of index 0 are not one.  PAD: the first
+// pass reads natural indices at or beyond pp.src_len as zeros (a zero-padded
+// input that is not stored).
+template <class SF, bool PAD>
 __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t blk, uint64_t* sm) {
-  constexpr uint32_t TILE_MAX = 1u << LOG_TILE;
+  constexpr uint32_t TILE_MAX = 1u << kSmallLogTile, THREADS = kSmallThreads;
   const uint32_t k = pp.k, c = pp.c, C = 1u << c;
-  const uint32_t tile = FULL ? TILE_MAX : 1u << (k + c);
+  const uint32_t tile = 1u << (k + c);
   const uint32_t tid = threadIdx.x;
   uint32_t hi_base = 0, m0 = 0, col0 = 0;
   if (pp.first) {
@@ -120,7 +102,7 @@ __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t bl
 #pragma unroll
   for (uint32_t q = 0; q < TILE_MAX / THREADS; q++) {
     const uint32_t e = tid + q * THREADS;
-    if (FULL || e < tile) {
+    if (e < tile) {
       const uint32_t col = e & (C - 1), row = e >> c;
       uint32_t g, t;
       if (pp.first) {
@@ -142,7 +124,7 @@ __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t bl
 #pragma unroll
     for (uint32_t q = 0; q < TILE_MAX / 2 / THREADS; q++) {
       const uint32_t b = tid + q * THREADS;
-      if (FULL || b < tile / 2) {
+      if (b < tile / 2) {
         const uint32_t col = b & (C - 1), t0 = (b >> c) << 1;
         const uint32_t jg = pp.first ? 0 : m0 + col;
         const uint32_t e0 = (t0 << c) | col, e1 = e0 + C;
@@ -164,7 +146,7 @@ __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t bl
 #pragma unroll
     for (uint32_t q = 0; q < TILE_MAX / 4 / THREADS; q++) {
       const uint32_t ga = tid + q * THREADS;
-      if (FULL || ga < tile / 4) {
+      if (ga < tile / 4) {
         const uint32_t col = ga & (C - 1), g = ga >> c;
         const uint32_t j = g & (h - 1);
         const uint32_t t0 = ((g >> (i - 1)) << (i + 1)) | j;
@@ -198,7 +180,7 @@ __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t bl
 #pragma unroll
   for (uint32_t q = 0; q < TILE_MAX / THREADS; q++) {
     const uint32_t e = tid + q * THREADS;
-    if (FULL || e < tile) {
+    if (e < tile) {
       const uint32_t col = e & (C - 1), row = e >> c;
       const uint32_t g = pp.first ? (rev_bits_small(col0 + col, xcols_log) << k) + row
                                   : hi_base + (row << pp.S) + m0 + col;
@@ -209,26 +191,71 @@ __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t bl
   }
 }
 
-template <class SF, int LOG_TILE, int THREADS, bool FULL>
-__global__ void __launch_bounds__(THREADS) small_pass_kernel(SmallPass pp) {
-  __shared__ uint64_t sm[1u << LOG_TILE];
-  small_pass_body<SF, LOG_TILE, THREADS, false, FULL>(pp, blockIdx.x, sm);
+template <class SF>
+__global__ void __launch_bounds__(kSmallThreads) small_pass_kernel(SmallPass pp) {
+  __shared__ uint64_t sm[1u << kSmallLogTile];
+  small_pass_body<SF, false>(pp, blockIdx.x, sm);
 }
 
 // The same pass over many columns of one size: column blockIdx.y reads
 // srcs[y] and writes dsts[y] (device pointer tables).
-template <class SF, int LOG_TILE, int THREADS, bool FULL>
-__global__ void __launch_bounds__(THREADS) small_pass_cols_kernel(SmallPass pp, const uint64_t* const* srcs,
-                                                                  uint64_t* const* dsts) {
-  __shared__ uint64_t sm[1u << LOG_TILE];
+template <class SF>
+__global__ void __launch_bounds__(kSmallThreads) small_pass_cols_kernel(SmallPass pp, const uint64_t* const* srcs,
+                                                                        uint64_t* const* dsts) {
+  __shared__ uint64_t sm[1u << kSmallLogTile];
   SmallPass q = pp;
   q.src = srcs[blockIdx.y];
   q.dst = dsts[blockIdx.y];
-  small_pass_body<SF, LOG_TILE, THREADS, true, FULL>(q, blockIdx.x, sm);
+  small_pass_body<SF, true>(q, blockIdx.x, sm);
 }
 
-// Flat table entry e = 2^s - 1 + j holds root^(j * 2^(log_n - 1 - s)), in
-// twiddle form, from three power tables pw[t][i] = root^(i * 1024^t).
+// Four CTAs per SM (64 registers, no spill): 2^24 Goldilocks forward 0.398 ms with
+// three and 0.382 with four (B200).
+template <class SF, int K, bool FIRST, bool INV>
+__global__ void __launch_bounds__(kTileThreads, 4)
+    small_tile_kernel(SmallPass pp, const uint64_t* const* srcs, uint64_t* const* dsts) {
+  using T = SmallTile<SF, K, FIRST, INV>;
+  __shared__ typename SF::word sm[T::kWords];
+  // A pass after the first is launched as the programmatic dependent of the one
+  // before it: its launch overlaps that pass's end.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  T(pp, srcs ? srcs[blockIdx.y] : pp.src, dsts ? dsts[blockIdx.y] : pp.dst, blockIdx.x, sm).run();
+}
+
+template <class SF, int K>
+static void launch_tile_k(const SmallPass& pp, dim3 grid, const uint64_t* const* srcs, uint64_t* const* dsts,
+                          cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kTileThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pp.first ? 0 : 1;
+  if (pp.first && pp.inverse) cudaLaunchKernelEx(&cfg, small_tile_kernel<SF, K, true, true>, pp, srcs, dsts);
+  else if (pp.first) cudaLaunchKernelEx(&cfg, small_tile_kernel<SF, K, true, false>, pp, srcs, dsts);
+  else if (pp.inverse) cudaLaunchKernelEx(&cfg, small_tile_kernel<SF, K, false, true>, pp, srcs, dsts);
+  else cudaLaunchKernelEx(&cfg, small_tile_kernel<SF, K, false, false>, pp, srcs, dsts);
+}
+
+// A pass on whole 2^12-element tiles; m columns when srcs and dsts are given.
+template <class SF>
+static void launch_tile(const SmallPass& pp, uint32_t m, const uint64_t* const* srcs, uint64_t* const* dsts,
+                        cudaStream_t st) {
+  const dim3 grid((unsigned)((1ull << pp.log_n) >> kTileLog), m);
+  switch (pp.k) {
+    case 6: launch_tile_k<SF, 6>(pp, grid, srcs, dsts, st); break;
+    case 7: launch_tile_k<SF, 7>(pp, grid, srcs, dsts, st); break;
+    case 8: launch_tile_k<SF, 8>(pp, grid, srcs, dsts, st); break;
+    case 9: launch_tile_k<SF, 9>(pp, grid, srcs, dsts, st); break;
+    default: launch_tile_k<SF, 10>(pp, grid, srcs, dsts, st); break;
+  }
+}
+
+// Flat table entry e = 2^s - 1 + j is that of root^(j * 2^(log_n - 1 - s)),
+// from three power tables pw[t][i] = root^(i * 1024^t).
 template <class SF>
 __global__ void small_twiddle_kernel(const uint64_t* __restrict__ pw, uint64_t* __restrict__ out, uint32_t log_n) {
   const uint64_t total = (1ull << log_n) - 1;
@@ -238,18 +265,30 @@ __global__ void small_twiddle_kernel(const uint64_t* __restrict__ pw, uint64_t* 
     const uint64_t j = e + 1 - (1ull << s);
     const uint64_t x = j << (log_n - 1 - s);
     uint64_t v = SF::mul(__ldg(pw + (x & 1023)), __ldg(pw + 1024 + ((x >> 10) & 1023)));
-    out[e] = SF::mul(v, __ldg(pw + 2048 + (x >> 20)));
+    out[e] = SF::entry(SF::mul(SF::mul(v, __ldg(pw + 2048 + (x >> 20))), 1));
   }
 }
 
-// out[i] = in[i] * f (f chosen by the caller): converts between canonical and
-// twiddle form (f = R^2 mod p, or the integer 1).  in and out may be the same
-// array (each element is read, then written, by one thread), so the pointers
-// are not restrict and the loads are coherent.
+// The three power tables of `base` the kernels expand: pw[1024 t + i] =
+// base^(i 1024^t), all in twiddle form, with pw[i] times c (twiddle form).
 template <class SF>
-__global__ void small_scale_kernel(const uint64_t* in, uint64_t* out, uint64_t count, uint64_t f) {
+__global__ void small_power_tables_kernel(uint64_t base, uint64_t one, uint64_t c, uint64_t* __restrict__ pw) {
+  const uint32_t t = blockIdx.x, i = threadIdx.x;
+  uint64_t b = base;
+  for (uint32_t k = 0; k < 10 * t; k++) b = SF::mul(b, b);
+  uint64_t r = t == 0 ? c : one;
+  for (uint32_t k = 0; k < 10; k++) {
+    if ((i >> k) & 1) r = SF::mul(r, b);
+    b = SF::mul(b, b);
+  }
+  pw[1024 * t + i] = r;
+}
+
+// Table entries <-> canonical values (in may be out).
+template <class SF>
+__global__ void small_entries_kernel(const uint64_t* in, uint64_t* out, uint64_t count, bool to_entries) {
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x)
-    out[i] = SF::mul(f, in[i]);
+    out[i] = to_entries ? SF::entry(in[i] % SF::P) : SF::entry_value(in[i]);
 }
 
 // out[i] = c * base^i for i < count (< 2^30), from power tables of base in
@@ -322,59 +361,48 @@ __global__ void small_bit_reverse_kernel(const uint64_t* __restrict__ src, uint6
 
 int grid_for(uint64_t count) { return (int)std::min<uint64_t>((count + 255) / 256, 148 * 16); }
 
-template <class SF, bool FULL>
-static void launch_small_pass_t(const SmallPass& pp, uint64_t tiles, cudaStream_t st) {
-  small_pass_kernel<SF, kSmallLogTile, kSmallThreads, FULL><<<(unsigned)tiles, kSmallThreads, 0, st>>>(pp);
-}
-
 cudaError_t launch_small_pass(int field, const SmallPass& pp, uint64_t tiles, cudaStream_t st) {
-  const bool full = pp.k + pp.c == (uint32_t)kSmallLogTile;
-  if (field == kGoldilocksField && pp.k + pp.c == (uint32_t)kSmallLogTileB) {
-    // a whole 2^11-element tile: the smaller CTA
-    small_pass_kernel<Goldilocks, kSmallLogTileB, kSmallThreadsB, true>
-        <<<(unsigned)tiles, kSmallThreadsB, 0, st>>>(pp);
-    return cudaGetLastError();
-  }
-  if (field == kGoldilocksField) {
-    if (full) launch_small_pass_t<Goldilocks, true>(pp, tiles, st);
-    else launch_small_pass_t<Goldilocks, false>(pp, tiles, st);
-  } else {
-    if (full) launch_small_pass_t<BabyBear, true>(pp, tiles, st);
-    else launch_small_pass_t<BabyBear, false>(pp, tiles, st);
-  }
+  if (field == kGoldilocksField) small_pass_kernel<Goldilocks><<<(unsigned)tiles, kSmallThreads, 0, st>>>(pp);
+  else small_pass_kernel<BabyBear><<<(unsigned)tiles, kSmallThreads, 0, st>>>(pp);
   return cudaGetLastError();
 }
 
 cudaError_t launch_small_pass_cols(int field, const SmallPass& pp, uint64_t tiles, uint32_t m,
                                    const uint64_t* const* srcs, uint64_t* const* dsts, cudaStream_t st) {
   const dim3 grid((unsigned)tiles, m);
-  const bool full = pp.k + pp.c == (uint32_t)kSmallLogTile;
-  if (field == kGoldilocksField && pp.k + pp.c == (uint32_t)kSmallLogTileB) {
-    small_pass_cols_kernel<Goldilocks, kSmallLogTileB, kSmallThreadsB, true>
-        <<<grid, kSmallThreadsB, 0, st>>>(pp, srcs, dsts);
-    return cudaGetLastError();
-  }
-  if (field == kGoldilocksField) {
-    if (full)
-      small_pass_cols_kernel<Goldilocks, kSmallLogTile, kSmallThreads, true><<<grid, kSmallThreads, 0, st>>>(pp, srcs, dsts);
-    else
-      small_pass_cols_kernel<Goldilocks, kSmallLogTile, kSmallThreads, false><<<grid, kSmallThreads, 0, st>>>(pp, srcs, dsts);
-  } else {
-    if (full)
-      small_pass_cols_kernel<BabyBear, kSmallLogTile, kSmallThreads, true><<<grid, kSmallThreads, 0, st>>>(pp, srcs, dsts);
-    else
-      small_pass_cols_kernel<BabyBear, kSmallLogTile, kSmallThreads, false><<<grid, kSmallThreads, 0, st>>>(pp, srcs, dsts);
-  }
+  if (field == kGoldilocksField)
+    small_pass_cols_kernel<Goldilocks><<<grid, kSmallThreads, 0, st>>>(pp, srcs, dsts);
+  else
+    small_pass_cols_kernel<BabyBear><<<grid, kSmallThreads, 0, st>>>(pp, srcs, dsts);
   return cudaGetLastError();
 }
 
-cudaError_t launch_small_scale(int field, const uint64_t* in, uint64_t* out, uint64_t count, uint64_t f,
-                               cudaStream_t st) {
+constexpr size_t kPowerTableBytes = (size_t)3 * 1024 * 8;
+
+// base and c canonical.
+cudaError_t launch_small_power_tables(int field, uint64_t base, uint64_t c, uint64_t* d_pw, cudaStream_t st) {
+  const SmallHost& H = small_host(field);
+  if (field == kGoldilocksField)
+    small_power_tables_kernel<Goldilocks><<<3, 1024, 0, st>>>(H.to_tw(base), H.to_tw(1), H.to_tw(c), d_pw);
+  else
+    small_power_tables_kernel<BabyBear><<<3, 1024, 0, st>>>(H.to_tw(base), H.to_tw(1), H.to_tw(c), d_pw);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_small_tile(int field, const SmallPass& pp, uint32_t m, const uint64_t* const* srcs,
+                              uint64_t* const* dsts, cudaStream_t st) {
+  if (field == kGoldilocksField) launch_tile<Goldilocks>(pp, m, srcs, dsts, st);
+  else launch_tile<BabyBear>(pp, m, srcs, dsts, st);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_small_entries(int field, const uint64_t* in, uint64_t* out, uint64_t count, bool to_entries,
+                                 cudaStream_t st) {
   if (count == 0) return cudaSuccess;
   if (field == kGoldilocksField)
-    small_scale_kernel<Goldilocks><<<grid_for(count), 256, 0, st>>>(in, out, count, f);
+    small_entries_kernel<Goldilocks><<<grid_for(count), 256, 0, st>>>(in, out, count, to_entries);
   else
-    small_scale_kernel<BabyBear><<<grid_for(count), 256, 0, st>>>(in, out, count, f);
+    small_entries_kernel<BabyBear><<<grid_for(count), 256, 0, st>>>(in, out, count, to_entries);
   return cudaGetLastError();
 }
 
@@ -384,14 +412,24 @@ struct SmallPlanPass {
   uint32_t S, k, c;
 };
 
-std::vector<SmallPlanPass> small_plan(uint32_t log_n, int field) {
-  std::vector<SmallPlanPass> plan;
-  const bool b = small_use_b(field, log_n);
-  const uint32_t lt = b ? kSmallLogTileB : kSmallLogTile;
-  const uint32_t kmax = b ? kSmallKmaxB : kSmallKmax;
+struct SmallPlan {
+  bool tiles = false;  // every pass on whole tiles of small_tile.cuh
+  std::vector<SmallPlanPass> passes;
+};
+
+// The passes of a transform of 2^log_n elements; `unit0`: the factors of index 0
+// are one (the inverse's always, and a table's whose entries 0 are).  From 2^12
+// on whole tiles, with passes of six to ten stages: a pass of ten exchanges
+// twice but saves a sweep (2^20 Goldilocks forward 0.0327 ms as 10 + 10 stages,
+// 0.0368 as 7 + 7 + 6; both are faster than this file's own passes at every size
+// from 2^12, 0.0143 ms against 0.0205 there, B200).
+SmallPlan small_plan(uint32_t log_n, bool unit0) {
+  SmallPlan plan;
   if (log_n == 0) return plan;
-  if (log_n <= lt) {
-    plan.push_back({0, log_n, 0});
+  plan.tiles = unit0 && log_n >= kTileLog;
+  const uint32_t lt = plan.tiles ? kTileLog : kSmallLogTile, kmax = plan.tiles ? kTileKmax : kSmallKmax;
+  if (log_n <= lt && !plan.tiles) {
+    plan.passes.push_back({0, log_n, 0});
     return plan;
   }
   const uint32_t P = (log_n + kmax - 1) / kmax;
@@ -401,7 +439,7 @@ std::vector<SmallPlanPass> small_plan(uint32_t log_n, int field) {
     uint32_t c = lt - k;
     const uint32_t lim = p == 0 ? log_n - k : S;
     if (c > lim) c = lim;
-    plan.push_back({S, k, c});
+    plan.passes.push_back({S, k, c});
     S += k;
   }
   return plan;
@@ -415,7 +453,7 @@ struct SmallTable {
   int field = 0;
   uint32_t log_n = 0;
   uint64_t root = 0;          // canonical; the key of root-derived tables
-  uint64_t* d_table = nullptr;  // 2^log_n - 1 entries in twiddle form (one when log_n == 0)
+  uint64_t* d_table = nullptr;  // 2^log_n - 1 entries (SF::entry; one when log_n == 0)
   size_t bytes = 0;
   int refs = 0;
   bool tw0_one = true;
@@ -514,25 +552,14 @@ int small_acquire(int field, uint32_t log_n, uint64_t root, SmallTable** out) {
     return cuda_fail(ce, "twiddle table");
   }
   if (log_n > 0) {
-    // pw[t][i] = root^(i * 1024^t), computed canonically, stored in twiddle form.
-    std::vector<uint64_t> pw(3 * 1024);
-    uint64_t step = root;
-    for (int t = 0; t < 3; t++) {
-      uint64_t cur = 1;
-      for (int i = 0; i < 1024; i++) {
-        pw[t * 1024 + i] = H.to_tw(cur);
-        cur = H.mul(cur, step);
-      }
-      step = H.pow(step, 1024);
-    }
     void* d_pw = nullptr;
-    int rc = pool_get(pw.size() * 8, &d_pw);
+    int rc = pool_get(kPowerTableBytes, &d_pw);
     if (rc) {
       cudaFree(e->d_table);
       delete e;
       return rc;
     }
-    ce = cudaMemcpyAsync(d_pw, pw.data(), pw.size() * 8, cudaMemcpyHostToDevice, c.stream);
+    ce = launch_small_power_tables(field, root, 1, (uint64_t*)d_pw, c.stream);
     const uint64_t total = small_entries(log_n);
     if (ce == cudaSuccess) {
       if (field == kGoldilocksField)
@@ -544,7 +571,7 @@ int small_acquire(int field, uint32_t log_n, uint64_t root, SmallTable** out) {
       ce = cudaGetLastError();
     }
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(c.stream);
-    pool_put(d_pw, pw.size() * 8);
+    pool_put(d_pw, kPowerTableBytes);
     if (ce != cudaSuccess) {
       cudaFree(e->d_table);
       delete e;
@@ -578,11 +605,11 @@ int small_upload_foreign(int field, uint32_t log_n, const zntt_stage* stages, Sm
     ce = cudaMemcpyAsync(e->d_table + (((size_t)1 << s) - 1), stages[s].ptr, ((size_t)1 << s) * 8,
                          cudaMemcpyHostToDevice, c.stream);
   }
-  // Canonical -> twiddle form: mul(x, R^2) = x * R.  Entries at or above p are
-  // reduced on the way (the reference's Fields are canonical already).
+  // Canonical values -> entries.  Values at or above p are reduced on the way
+  // (the reference's Fields are canonical already).
   if (ce == cudaSuccess)
-    ce = launch_small_scale(field, e->d_table, e->d_table, small_entries(log_n) - (log_n == 0 ? 1 : 0),
-                            H.mul(H.r, H.r), c.stream);
+    ce = launch_small_entries(field, e->d_table, e->d_table, small_entries(log_n) - (log_n == 0 ? 1 : 0), true,
+                              c.stream);
   if (ce != cudaSuccess) {
     cudaStreamSynchronize(c.stream);
     cudaFree(e->d_table);
@@ -617,24 +644,28 @@ SmallRegistration* small_find_registration(int field, uint32_t log_n, const zntt
 // src_len) and writes dsts[y]; the later passes run in place on dsts[y], so no
 // scratch is needed.  At least one pass (log_n >= 1).
 int small_run_cols(const SmallTable* t, uint32_t m, const uint64_t* const* srcs, uint64_t* const* dsts,
-                   uint32_t src_len, bool inverse, bool scale, uint64_t scale_tw, cudaStream_t st) {
-  const std::vector<SmallPlanPass> plan = small_plan(t->log_n, t->field);
-  for (size_t p = 0; p < plan.size(); p++) {
+                   uint32_t src_len, bool inverse, bool scale, uint64_t scale_tw, cudaStream_t st,
+                   const uint64_t* coset_pw = nullptr) {
+  const SmallPlan plan = small_plan(t->log_n, inverse || t->tw0_one);
+  for (size_t p = 0; p < plan.passes.size(); p++) {
     SmallPass pp;
     std::memset(&pp, 0, sizeof(pp));
     pp.tw = t->d_table;
     pp.log_n = t->log_n;
-    pp.S = plan[p].S;
-    pp.k = plan[p].k;
-    pp.c = plan[p].c;
+    pp.S = plan.passes[p].S;
+    pp.k = plan.passes[p].k;
+    pp.c = plan.passes[p].c;
     pp.first = p == 0;
     pp.inverse = inverse;
     pp.tw0_one = t->tw0_one;
-    pp.scale = p + 1 == plan.size() && scale;
+    const bool last = p + 1 == plan.passes.size();
+    pp.scale = last && scale;
     pp.scale_val = scale_tw;
+    pp.coset_pw = last ? coset_pw : nullptr;  // whole tiles only
     pp.src_len = src_len;
     const uint64_t tiles = (1ull << t->log_n) >> (pp.k + pp.c);
-    cudaError_t ce = launch_small_pass_cols(t->field, pp, tiles, m, p == 0 ? srcs : dsts, dsts, st);
+    cudaError_t ce = plan.tiles ? launch_small_tile(t->field, pp, m, p == 0 ? srcs : dsts, dsts, st)
+                                : launch_small_pass_cols(t->field, pp, tiles, m, p == 0 ? srcs : dsts, dsts, st);
     if (ce != cudaSuccess) return cuda_fail(ce, "small-field pass");
   }
   return ZNTT_OK;
@@ -642,33 +673,36 @@ int small_run_cols(const SmallTable* t, uint32_t m, const uint64_t* const* srcs,
 
 int small_run(const SmallTable* t, const uint64_t* src, uint64_t* dst, uint64_t* scratch, bool inverse, bool scale,
               uint64_t scale_tw, cudaStream_t st) {
-  const std::vector<SmallPlanPass> plan = small_plan(t->log_n, t->field);
-  if (plan.empty()) {  // one element: a copy (the 1/n scale is by one)
+  const SmallPlan plan = small_plan(t->log_n, inverse || t->tw0_one);
+  const size_t np = plan.passes.size();
+  if (np == 0) {  // one element: a copy (the 1/n scale is by one)
     if (src != dst) {
       cudaError_t ce = cudaMemcpyAsync(dst, src, 8, cudaMemcpyDeviceToDevice, st);
       if (ce != cudaSuccess) return cuda_fail(ce, "copy");
     }
     return ZNTT_OK;
   }
-  uint64_t* mid = (src == dst && plan.size() > 1) ? scratch : dst;
-  for (size_t p = 0; p < plan.size(); p++) {
-    const bool first = p == 0, last = p + 1 == plan.size();
+  uint64_t* mid = (src == dst && np > 1) ? scratch : dst;
+  for (size_t p = 0; p < np; p++) {
+    const bool first = p == 0, last = p + 1 == np;
     SmallPass pp;
     std::memset(&pp, 0, sizeof(pp));
     pp.src = first ? src : mid;
     pp.dst = last ? dst : mid;
     pp.tw = t->d_table;
     pp.log_n = t->log_n;
-    pp.S = plan[p].S;
-    pp.k = plan[p].k;
-    pp.c = plan[p].c;
+    pp.S = plan.passes[p].S;
+    pp.k = plan.passes[p].k;
+    pp.c = plan.passes[p].c;
+    pp.src_len = (uint32_t)(1ull << t->log_n);
     pp.first = first;
     pp.inverse = inverse;
     pp.tw0_one = t->tw0_one;
     pp.scale = last && scale;
     pp.scale_val = scale_tw;
     const uint64_t tiles = (1ull << t->log_n) >> (pp.k + pp.c);
-    cudaError_t ce = launch_small_pass(t->field, pp, tiles, st);
+    cudaError_t ce = plan.tiles ? launch_small_tile(t->field, pp, 1, nullptr, nullptr, st)
+                                : launch_small_pass(t->field, pp, tiles, st);
     if (ce != cudaSuccess) return cuda_fail(ce, "small-field pass");
   }
   return ZNTT_OK;
@@ -805,7 +839,7 @@ int small_precompute(int field, size_t log_n, const uint64_t* root, uint64_t* co
   SmallTable* t = nullptr;
   rc = small_acquire(field, (uint32_t)log_n, root[0] % H.p, &t);
   if (rc) return rc;
-  // Twiddle form -> canonical (mul by canonical one), then download by stage.
+  // Table entries -> canonical values, then download by stage.
   const size_t entries = small_entries((uint32_t)log_n);
   void* canon = nullptr;
   rc = pool_get(entries * 8, &canon);
@@ -813,7 +847,7 @@ int small_precompute(int field, size_t log_n, const uint64_t* root, uint64_t* co
     small_release(t);
     return rc;
   }
-  cudaError_t ce = launch_small_scale(field, t->d_table, (uint64_t*)canon, entries, 1, c.stream);
+  cudaError_t ce = launch_small_entries(field, t->d_table, (uint64_t*)canon, entries, false, c.stream);
   for (size_t s = 0; s < log_n && ce == cudaSuccess; s++)
     ce = cudaMemcpyAsync(stage_out[s], (uint64_t*)canon + (((size_t)1 << s) - 1), ((size_t)1 << s) * 8,
                          cudaMemcpyDeviceToHost, c.stream);
@@ -930,7 +964,7 @@ int small_ntt_device(const zntt_twiddles* tw, const uint64_t* d_src, uint64_t* d
   const bool inverse = mode == ZNTT_INVERSE;
   const uint64_t ninv = n_inverse_tw(H, t->log_n);
   cudaStream_t st = stream ? (cudaStream_t)stream : c.stream;
-  const bool need_scratch = d_src == d_dst && small_plan(t->log_n, t->field).size() > 1;
+  const bool need_scratch = d_src == d_dst && small_plan(t->log_n, inverse || t->tw0_one).passes.size() > 1;
   if (need_scratch && !d_scratch) {
     const size_t bytes = ((size_t)8) << t->log_n;
     void* s = nullptr;
@@ -956,21 +990,10 @@ std::map<std::pair<int, uint32_t>, uint64_t*>& small_fold_tables() {
 // c * base^i (i < count) on the device: in twiddle form when c is given in
 // twiddle form, canonical when c is the plain integer 1.
 int small_powers(int field, uint64_t base, uint64_t c, uint64_t* out, uint64_t count, cudaStream_t st) {
-  const SmallHost& H = small_host(field);
-  std::vector<uint64_t> pw(3 * 1024);
-  uint64_t step = base % H.p;
-  for (int t = 0; t < 3; t++) {
-    uint64_t cur = 1;
-    for (int i = 0; i < 1024; i++) {
-      pw[t * 1024 + i] = H.to_tw(cur);
-      cur = H.mul(cur, step);
-    }
-    step = H.pow(step, 1024);
-  }
   void* d_pw = nullptr;
-  int rc = pool_get(pw.size() * 8, &d_pw);
+  int rc = pool_get(kPowerTableBytes, &d_pw);
   if (rc) return rc;
-  cudaError_t ce = cudaMemcpyAsync(d_pw, pw.data(), pw.size() * 8, cudaMemcpyHostToDevice, st);
+  cudaError_t ce = launch_small_power_tables(field, base, 1, (uint64_t*)d_pw, st);
   if (ce == cudaSuccess && count) {
     if (field == kGoldilocksField)
       small_powers_kernel<Goldilocks><<<grid_for(count), 256, 0, st>>>((const uint64_t*)d_pw, c, out, count);
@@ -979,7 +1002,7 @@ int small_powers(int field, uint64_t base, uint64_t c, uint64_t* out, uint64_t c
     ce = cudaGetLastError();
   }
   cudaError_t ce2 = cudaStreamSynchronize(st);  // the power tables return to the pool
-  pool_put(d_pw, pw.size() * 8);
+  pool_put(d_pw, kPowerTableBytes);
   if (ce == cudaSuccess) ce = ce2;
   if (ce != cudaSuccess) return cuda_fail(ce, "powers");
   return ZNTT_OK;
@@ -1107,18 +1130,8 @@ int small_coset_lde_many(const zntt_twiddles* tw_in, const zntt_twiddles* tw_out
   Context& c = ctx();
   std::lock_guard<std::recursive_mutex> lock(c.mu);
   cudaStream_t st = stream ? (cudaStream_t)stream : c.stream;
-  std::vector<uint64_t> pw(3 * 1024);
-  uint64_t step = shift[0];
-  for (int t = 0; t < 3; t++) {
-    uint64_t cur = 1;
-    for (int i = 0; i < 1024; i++) {
-      pw[t * 1024 + i] = H.to_tw(cur);
-      cur = H.mul(cur, step);
-    }
-    step = H.pow(step, 1024);
-  }
   void* d_pw = nullptr;
-  int rc = pool_get(pw.size() * 8, &d_pw);
+  int rc = pool_get(kPowerTableBytes, &d_pw);
   if (rc) return rc;
   if (ti->log_n >= 1 && m <= 65535) {
     // All columns per launch: the inverse transforms into a contiguous buffer of
@@ -1132,7 +1145,7 @@ int small_coset_lde_many(const zntt_twiddles* tw_in, const zntt_twiddles* tw_out
     if (!rc) rc = pool_get(tab_bytes, &tabs);
     if (rc) {
       if (tmp) pool_put(tmp, tmp_bytes);
-      pool_put(d_pw, pw.size() * 8);
+      pool_put(d_pw, kPowerTableBytes);
       return rc;
     }
     std::vector<const void*> h(3 * (size_t)m);
@@ -1144,23 +1157,30 @@ int small_coset_lde_many(const zntt_twiddles* tw_in, const zntt_twiddles* tw_out
     const uint64_t* const* t_src = static_cast<const uint64_t* const*>(tabs);
     uint64_t* const* t_tmp = static_cast<uint64_t* const*>(tabs) + m;
     uint64_t* const* t_out = static_cast<uint64_t* const*>(tabs) + 2 * (size_t)m;
-    cudaError_t ce = cudaMemcpyAsync(d_pw, pw.data(), pw.size() * 8, cudaMemcpyHostToDevice, st);
+    // On whole tiles the inverse's last pass scales by n^-1 shift^i (n^-1 in the
+    // first power table); else the inverse scales by n^-1 and a launch of its own
+    // by shift^i.
+    const bool fused = small_plan(ti->log_n, true).tiles;
+    const uint64_t n_inv = H.inv(n_in % H.p);
+    cudaError_t ce = launch_small_power_tables(ti->field, shift[0], fused ? n_inv : 1, (uint64_t*)d_pw, st);
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(tabs, h.data(), tab_bytes, cudaMemcpyHostToDevice, st);
     if (ce == cudaSuccess) {
-      rc = small_run_cols(ti, m, t_src, t_tmp, (uint32_t)n_in, true, true, n_inverse_tw(H, ti->log_n), st);
+      rc = small_run_cols(ti, m, t_src, t_tmp, (uint32_t)n_in, true, !fused, H.to_tw(n_inv), st,
+                          fused ? (const uint64_t*)d_pw : nullptr);
       if (rc == ZNTT_OK) {
-        if (ti->field == kGoldilocksField)
-          small_coset_scale_cols_kernel<Goldilocks><<<grid_for((uint64_t)m * n_in), 256, 0, st>>>(
-              (const uint64_t*)d_pw, static_cast<uint64_t*>(tmp), (uint64_t)m * n_in, ti->log_n);
-        else
-          small_coset_scale_cols_kernel<BabyBear><<<grid_for((uint64_t)m * n_in), 256, 0, st>>>(
-              (const uint64_t*)d_pw, static_cast<uint64_t*>(tmp), (uint64_t)m * n_in, ti->log_n);
+        const uint64_t total = (uint64_t)m * n_in;
+        if (!fused && ti->field == kGoldilocksField)
+          small_coset_scale_cols_kernel<Goldilocks><<<grid_for(total), 256, 0, st>>>(
+              (const uint64_t*)d_pw, static_cast<uint64_t*>(tmp), total, ti->log_n);
+        else if (!fused)
+          small_coset_scale_cols_kernel<BabyBear><<<grid_for(total), 256, 0, st>>>(
+              (const uint64_t*)d_pw, static_cast<uint64_t*>(tmp), total, ti->log_n);
         ce = cudaGetLastError();
         if (ce == cudaSuccess) rc = small_run_cols(to, m, t_tmp, t_out, (uint32_t)n_in, false, false, 0, st);
       }
     }
     cudaError_t ce2 = cudaStreamSynchronize(st);  // the buffers return to the pool after the stream is done
-    pool_put(d_pw, pw.size() * 8);
+    pool_put(d_pw, kPowerTableBytes);
     pool_put(tmp, tmp_bytes);
     pool_put(tabs, tab_bytes);
     if (rc) return rc;
@@ -1172,13 +1192,13 @@ int small_coset_lde_many(const zntt_twiddles* tw_in, const zntt_twiddles* tw_out
   const size_t sbytes = (size_t)8 << to->log_n;
   rc = pool_get(sbytes, &scratch);
   if (rc) {
-    pool_put(d_pw, pw.size() * 8);
+    pool_put(d_pw, kPowerTableBytes);
     return rc;
   }
   // One stream: the columns run one after another and share the power tables and
   // the forward transform's scratch (one-element inputs, or more columns than a
   // launch's second grid dimension holds).
-  cudaError_t ce = cudaMemcpyAsync(d_pw, pw.data(), pw.size() * 8, cudaMemcpyHostToDevice, st);
+  cudaError_t ce = launch_small_power_tables(ti->field, shift[0], 1, (uint64_t*)d_pw, st);
   for (uint32_t k = 0; k < m && ce == cudaSuccess && rc == ZNTT_OK; k++) {
     uint64_t* out = d_out[k];
     rc = small_run(ti, d_evals[k], out, nullptr, true, true, n_inverse_tw(H, ti->log_n), st);  // out of place
@@ -1193,7 +1213,7 @@ int small_coset_lde_many(const zntt_twiddles* tw_in, const zntt_twiddles* tw_out
   }
   // The power tables and the scratch return to the pool after the stream is done.
   cudaError_t ce2 = cudaStreamSynchronize(st);
-  pool_put(d_pw, pw.size() * 8);
+  pool_put(d_pw, kPowerTableBytes);
   pool_put(scratch, sbytes);
   if (rc) return rc;
   if (ce == cudaSuccess) ce = ce2;

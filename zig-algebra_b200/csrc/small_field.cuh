@@ -8,7 +8,9 @@
 // R = 1 for Goldilocks (a direct reduction) and R = 2^32 for BabyBear (a 32-bit
 // Montgomery reduction).  Twiddles and scale factors are kept in "twiddle
 // form" w * R mod p, so mul(w_form, x) = w * x mod p stays canonical, and
-// mul of two twiddle-form values is the twiddle form of their product.
+// mul of two twiddle-form values is the twiddle form of their product.  The
+// transforms' tables hold entries made from canonical factors (entry), which
+// mul_entry multiplies by.
 // Canonical values are unique, so results equal the reference's bit for bit.
 #pragma once
 
@@ -22,6 +24,13 @@ static __constant__ uint32_t kOpaqueOne = 1;
 
 struct Goldilocks {
   static constexpr int kId = 2;
+  using word = uint64_t;
+  // Table entries: the factors themselves.
+  static constexpr uint64_t kOneEntry = 1;
+  __device__ __forceinline__ static uint64_t entry(uint64_t w) { return w; }
+  __device__ __forceinline__ static uint64_t entry_value(uint64_t e) { return e; }
+  __device__ __forceinline__ static uint64_t neg_entry(uint64_t e) { return neg(e); }
+  __device__ __forceinline__ static uint64_t mul_entry(uint64_t e, uint64_t x) { return mul(e, x); }
   static constexpr uint64_t P = 0xFFFFFFFF00000001ull;
   static constexpr uint64_t EPS = 0xFFFFFFFFull;  // 2^64 mod p = 2^32 - 1
 
@@ -32,16 +41,6 @@ struct Goldilocks {
   // subtractions and selects stay on the ALU).
   __device__ __forceinline__ static uint64_t join(uint32_t lo, uint32_t hi) {
     return ((uint64_t)hi << 32) | lo;
-  }
-  // x - p when x >= p, else x, for x = (hi:lo) below 2^64.
-  __device__ __forceinline__ static uint64_t reduce_once(uint32_t lo, uint32_t hi) {
-    uint32_t d0, d1, br;
-    asm("sub.cc.u32  %0, %3, 1;\n\t"
-        "subc.cc.u32 %1, %4, 0xFFFFFFFF;\n\t"
-        "subc.u32    %2, 0, 0;"
-        : "=r"(d0), "=r"(d1), "=r"(br)
-        : "r"(lo), "r"(hi));
-    return br ? join(lo, hi) : join(d0, d1);
   }
   // a + b < 2p: the 65-bit sum less p, unless that borrows.
   __device__ __forceinline__ static uint64_t add(uint64_t a, uint64_t b) {
@@ -74,6 +73,45 @@ struct Goldilocks {
     return join(d0, d1);
   }
   __device__ __forceinline__ static uint64_t neg(uint64_t a) { return a == 0 ? 0 : P - a; }
+  // [0, 2^64) -> [0, p): a - p unless that borrows.
+  __device__ __forceinline__ static uint64_t canonical(uint64_t a) {
+    const uint32_t lo = (uint32_t)a, hi = (uint32_t)(a >> 32);
+    uint32_t d0, d1, br;
+    asm("sub.cc.u32  %0, %3, 1;\n\t"
+        "subc.cc.u32 %1, %4, 0xFFFFFFFF;\n\t"
+        "subc.u32    %2, 0, 0;"
+        : "=r"(d0), "=r"(d1), "=r"(br)
+        : "r"(lo), "r"(hi));
+    return br ? join(lo, hi) : join(d0, d1);
+  }
+  // The butterflies' u + t and u - t for t in [0, p) and any u below 2^64: the
+  // carry is worth 2^64 = 2^32 - 1, and adding (or taking) that cannot carry
+  // again, so the results are below 2^64 and congruent, not reduced.
+  __device__ __forceinline__ static void butterfly(uint64_t u, uint64_t t, uint64_t& sum, uint64_t& diff) {
+    const uint32_t u0 = (uint32_t)u, u1 = (uint32_t)(u >> 32), t0 = (uint32_t)t, t1 = (uint32_t)(t >> 32);
+    const uint32_t one = kOpaqueOne;
+    uint32_t s0, s1, c, d0, d1, b;
+    asm("mad.lo.cc.u32  %0, %3, %7, %5;\n\t"
+        "madc.lo.cc.u32 %1, %4, %7, %6;\n\t"
+        "addc.u32       %2, 0, 0;"
+        : "=r"(s0), "=r"(s1), "=r"(c)
+        : "r"(u0), "r"(u1), "r"(t0), "r"(t1), "r"(one));
+    asm("add.cc.u32  %0, %0, %2;\n\t"
+        "addc.u32    %1, %1, 0;"
+        : "+r"(s0), "+r"(s1)
+        : "r"(0u - c));
+    asm("sub.cc.u32  %0, %3, %5;\n\t"
+        "subc.cc.u32 %1, %4, %6;\n\t"
+        "subc.u32    %2, 0, 0;"
+        : "=r"(d0), "=r"(d1), "=r"(b)
+        : "r"(u0), "r"(u1), "r"(t0), "r"(t1));
+    asm("sub.cc.u32  %0, %0, %2;\n\t"
+        "subc.u32    %1, %1, 0;"
+        : "+r"(d0), "+r"(d1)
+        : "r"(b));
+    sum = join(s0, s1);
+    diff = join(d0, d1);
+  }
   // a * b mod p.  The 128-bit product is z3:z2:z1:z0 (32-bit words); with
   // 2^64 = 2^32 - 1 and 2^96 = -1 (mod p) it is (z1:z0) + z2 * 2^32 - z2 - z3.
   // That sum is c * 2^64 + t with c in {-1, 0, 1}; c * 2^64 = c * (2^32 - 1),
@@ -111,7 +149,7 @@ struct Goldilocks {
         "addc.u32    %1, %1, %3;"
         : "+r"(t0), "+r"(t1)
         : "r"(0u - c), "r"((uint32_t)((int32_t)c >> 31)));
-    return reduce_once(t0, t1);
+    return canonical(join(t0, t1));
   }
 };
 
@@ -128,6 +166,26 @@ struct BabyBear {
   static constexpr uint64_t P = 0x78000001ull;
   static constexpr uint32_t P32 = 0x78000001u;
   static constexpr uint32_t N0 = 0u - inverse_mod_2_32(P32);  // -p^-1 mod 2^32
+  using word = uint32_t;
+
+  // Table entries: a factor w (canonical) in the low half and its quotient
+  // q = floor(w 2^32 / p) in the high one.  For any x < 2^32 the quotient of
+  // x w by p is floor(x q / 2^32) or one more, so x w - floor(x q / 2^32) p is
+  // below 2p < 2^32 and needs only low products (Shoup's method): three
+  // multiplies where the Montgomery product takes two full ones and one low.
+  static constexpr uint64_t kOneEntry = 1 | (((1ull << 32) / P32) << 32);
+  __device__ __forceinline__ static uint64_t entry(uint64_t w) { return w | (((w << 32) / P32) << 32); }
+  __device__ __forceinline__ static uint64_t entry_value(uint64_t e) { return (uint32_t)e; }
+  // p - w and its quotient: floor((p - w) 2^32 / p) = 2^32 - 1 - q for w > 0; for
+  // w = 0 the pair (p, 2^32 - 1) multiplies to 0 as well.
+  __device__ __forceinline__ static uint64_t neg_entry(uint64_t e) {
+    return ((uint64_t)(~(uint32_t)(e >> 32)) << 32) | (P32 - (uint32_t)e);
+  }
+  __device__ __forceinline__ static uint64_t mul_entry(uint64_t e, uint64_t x) {
+    const uint32_t q = __umulhi((uint32_t)x, (uint32_t)(e >> 32));
+    const uint32_t r = (uint32_t)x * (uint32_t)e - q * P32;
+    return min(r, r - P32);
+  }
 
   // s < 2p: min(s, s - p) is s - p when s >= p and s otherwise (s - p wraps above s).
   __device__ __forceinline__ static uint64_t add(uint64_t a, uint64_t b) {
@@ -143,6 +201,11 @@ struct BabyBear {
     return min(d, dp);
   }
   __device__ __forceinline__ static uint64_t neg(uint64_t a) { return a == 0 ? 0 : P - a; }
+  __device__ __forceinline__ static uint64_t canonical(uint64_t a) { return a; }
+  __device__ __forceinline__ static void butterfly(uint32_t u, uint32_t t, uint32_t& sum, uint32_t& diff) {
+    sum = (uint32_t)add(u, t);
+    diff = (uint32_t)sub(u, t);
+  }
   // Montgomery: z = a * b < p^2; m = z * N0 mod 2^32; (z + m p) / 2^32 < 2p.
   __device__ __forceinline__ static uint64_t mul(uint64_t a, uint64_t b) {
     const uint64_t z = (uint64_t)(uint32_t)a * (uint32_t)b;
