@@ -18,6 +18,7 @@
 #include "field.cuh"
 #include "merkle_tree.cuh"
 #include "runtime.hpp"
+#include "shoup.cuh"
 #include "small.hpp"
 #include "small_field.cuh"
 
@@ -93,12 +94,10 @@ struct WideFoldLeafSource {
   const uint4* tab;
   uint64_t h;
   uint32_t stride;
-  fe half_inv, alpha;
+  fe_pair alpha;
   __device__ __forceinline__ fe fold(uint64_t m) const {
     const fe a = fe_load_nc(prev + 2 * m), b = fe_load_nc(prev + 2 * (m + 2 * h));
-    const fe even = fe_mul<F>(fe_add<F>(a, b), half_inv);
-    const fe odd = fe_mul<F>(fe_sub<F>(a, b), fe_load_nc(tab + 2 * (m << stride)));
-    return fe_add<F>(even, fe_mul<F>(alpha, odd));
+    return fe_fold<F>(a, b, tab + 4 * (m << stride), alpha);
   }
   __device__ __forceinline__ void get(uint64_t j, uint32_t (&d)[8], uint32_t one) const {
     const fe x = fold(j), y = fold(j + h);
@@ -307,19 +306,18 @@ extern "C" int zntt_fri_fold_commit(int field, const uint64_t* d_layer, uint32_t
     }
   } else {
     const void* tab = nullptr;
-    fe hv, av;
-    int rc = wide_fold_params(field, log_table, &tab, hv.v);
+    fe_pair av;
+    int rc = wide_fold_params(field, log_table, alpha, &tab, reinterpret_cast<uint64_t*>(&av));
     if (rc) return rc;
-    std::memcpy(av.v, alpha, 32);
     const uint4* prev = reinterpret_cast<const uint4*>(d_layer);
     uint4* next = reinterpret_cast<uint4*>(d_out);
     const uint4* t4 = reinterpret_cast<const uint4*>(tab);
     ce = cudaMemsetAsync(nodes, 0, 32, st);
     if (ce == cudaSuccess) {
       if (field == kBn254Fr)
-        ce = build_tree(WideFoldLeafSource<Bn254Fr>{prev, next, t4, h, stride, hv, av}, nodes, h, st);
+        ce = build_tree(WideFoldLeafSource<Bn254Fr>{prev, next, t4, h, stride, av}, nodes, h, st);
       else
-        ce = build_tree(WideFoldLeafSource<Bls12381Fr>{prev, next, t4, h, stride, hv, av}, nodes, h, st);
+        ce = build_tree(WideFoldLeafSource<Bls12381Fr>{prev, next, t4, h, stride, av}, nodes, h, st);
     }
   }
   if (ce == cudaSuccess && root_out) {

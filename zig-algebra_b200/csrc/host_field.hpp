@@ -119,6 +119,25 @@ struct HostField {
     mul(v, r2, r);
   }
 
+  // The fixed factor (shoup.cuh) of a Montgomery-form scalar t: its Montgomery
+  // reduction's row multipliers are the quotient, its result the plain value.
+  void fixed_factor(const uint64_t* t, uint64_t* w, uint64_t* q) const {
+    uint64_t a[4] = {t[0], t[1], t[2], t[3]};
+    while (geq(a, p)) sub_p(a);
+    for (int i = 0; i < 4; i++) {
+      const uint64_t m = a[0] * n0;
+      q[i] = m;
+      uint64_t c = 0;
+      for (int j = 0; j < 4; j++) {
+        u128 z = (u128)m * p[j] + a[j] + c;
+        if (j > 0) a[j - 1] = (uint64_t)z;
+        c = (uint64_t)(z >> 64);
+      }
+      a[3] = c;  // the value stays below p + 2^192
+    }
+    std::memcpy(w, a, 32);
+  }
+
   bool is_one(const uint64_t* a) const { return std::memcmp(a, one, 32) == 0; }
 };
 

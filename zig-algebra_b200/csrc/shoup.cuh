@@ -337,6 +337,21 @@ __device__ __forceinline__ fe pair_entry(const fe& q) {
   return low_merge(s);
 }
 
+// x / 2 mod p for x in [0, p): x or x + p, whichever is even, shifted down.
+template <class F>
+__device__ __forceinline__ fe fe_half(const fe& x) {
+  const uint32_t odd = 0u - (x.v[0] & 1u);
+  fe p;
+  p.v[0] = F::P0 & odd; p.v[1] = F::P1 & odd; p.v[2] = F::P2 & odd; p.v[3] = F::P3 & odd;
+  p.v[4] = F::P4 & odd; p.v[5] = F::P5 & odd; p.v[6] = F::P6 & odd; p.v[7] = F::P7 & odd;
+  const fe s = fe_add_raw(x, p);  // below 2p < 2^256
+  fe r;
+#pragma unroll
+  for (int k = 0; k < 7; k++) r.v[k] = __funnelshift_r(s.v[k], s.v[k + 1], 1);
+  r.v[7] = s.v[7] >> 1;
+  return r;
+}
+
 // k * p for k = 0..5, as two planes of 16-byte halves.
 struct Multiples {
   uint32_t h[2][6][4];
@@ -403,6 +418,21 @@ __device__ __forceinline__ void fe_butterfly(const fe& u, const fe& t, fe& sum, 
   }
   sum = fe_add_raw(u, t);
   diff = fe_sub_raw(fe_add_raw(u, off), t);
+}
+
+// One FRI fold: (a + b) / 2 + alpha (a - b) / (2 x) for canonical a and b, with the
+// fixed factors 1 / (2 x) (in memory) and alpha.
+template <class F>
+__device__ __forceinline__ fe fe_fold(const fe& a, const fe& b, const uint4* half_inv_x, const fe_pair& alpha) {
+  const fe even = fe_half<F>(fe_add<F>(a, b));
+  fe p;
+  p.v[0] = F::P0; p.v[1] = F::P1; p.v[2] = F::P2; p.v[3] = F::P3;
+  p.v[4] = F::P4; p.v[5] = F::P5; p.v[6] = F::P6; p.v[7] = F::P7;
+  const fe d = fe_sub_raw(fe_add_raw(a, p), b);  // (0, 2p)
+  const fe t = fe_mul_fixed<F>(d, ld_fe32(half_inv_x), ld_fe32(half_inv_x + 2));
+  const fe odd = fe_mul_fixed<F>(t, alpha.w, alpha.q);  // below 2p
+  if constexpr (F::kLazy) return fe_canonical<F>(fe_add_raw(even, odd));
+  else return fe_add<F>(even, fe_reduce<F>(odd));
 }
 
 }  // namespace zntt

@@ -31,9 +31,10 @@ int small_fri_fold(int field, const uint64_t* d_layer, uint32_t log_n, const uin
                    uint32_t log_table, void* stream);
 int small_fold_params(int field, uint32_t log_table, const uint64_t* alpha, const uint64_t** tab_out,
                       uint64_t* half_inv_tw, uint64_t* alpha_tw);
-// The 256-bit fields' fold constants (fri.cu): the resident table g^-j / 2 and 1/2
-// (Montgomery limbs as eight 32-bit words).
-int wide_fold_params(int field, uint32_t log_table, const void** tab_out, uint32_t half_inv[8]);
+// The 256-bit fields' fold constants (fri.cu): the resident table g^-j / 2 and alpha,
+// both as fixed factors (shoup.cuh).
+int wide_fold_params(int field, uint32_t log_table, const uint64_t* alpha, const void** tab_out,
+                     uint64_t alpha_factor[8]);
 int small_poly_mul(int field, const uint64_t* a, size_t a_len, const uint64_t* b, size_t b_len, size_t max_degree,
                    uint64_t* out, int64_t* out_degree);
 int small_ntt_columns(const zntt_twiddles* tw, const uint64_t* const* d_src, uint64_t* const* d_dst, uint32_t m,
