@@ -26,9 +26,8 @@ namespace zntt {
 namespace {
 
 // Two products by fixed factors and a halving: 428 multiply-pipe slots against
-// three Montgomery products' 816 (2^24 -> 2^23 BN254-Fr 0.419 -> 0.237 ms,
-// B200), and 192 bytes
-// from memory, which is then the closer bound.
+// three Montgomery products' 816, and 160 bytes of memory traffic, the two bounds
+// about equal (2^24 -> 2^23 BN254-Fr 0.419 -> 0.237 ms, B200).
 template <class F>
 __global__ void fri_fold_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, const uint4* __restrict__ tab,
                                 uint64_t half, uint32_t stride, fe_pair alpha) {

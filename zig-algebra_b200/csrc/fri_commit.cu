@@ -200,22 +200,11 @@ extern "C" int zntt_fri_commit_layer(int field, const uint64_t* d_layer, uint32_
   std::lock_guard<std::recursive_mutex> lock(c.mu);
   cudaStream_t st = stream ? (cudaStream_t)stream : c.stream;
   uint4* nodes = reinterpret_cast<uint4*>(d_nodes);
-  cudaError_t ce = cudaMemsetAsync(nodes, 0, 32, st);  // node 0 is unused and zero
-  if (ce == cudaSuccess) {
-    const uint4* wide = reinterpret_cast<const uint4*>(d_layer);
-    if (field == kBn254Fr)
-      ce = build_tree(WideLeafSource<Bn254Fr>{wide, h}, nodes, h, st);
-    else if (field == kBls12381Fr)
-      ce = build_tree(WideLeafSource<Bls12381Fr>{wide, h}, nodes, h, st);
-    else
-      ce = build_tree(SmallLeafSource{d_layer, h, field == kGoldilocksField ? 8u : 4u}, nodes, h, st);
-  }
-  if (ce == cudaSuccess && root_out) {
-    ce = cudaMemcpyAsync(root_out, d_nodes + 32, 32, cudaMemcpyDeviceToHost, st);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-  }
-  if (ce != cudaSuccess) return cuda_fail(ce, "fri layer commitment");
-  return ZNTT_OK;
+  const uint4* wide = reinterpret_cast<const uint4*>(d_layer);
+  const char* what = "fri layer commitment";
+  if (field == kBn254Fr) return commit_tree(WideLeafSource<Bn254Fr>{wide, h}, nodes, h, root_out, st, what);
+  if (field == kBls12381Fr) return commit_tree(WideLeafSource<Bls12381Fr>{wide, h}, nodes, h, root_out, st, what);
+  return commit_tree(SmallLeafSource{d_layer, h, field == kGoldilocksField ? 8u : 4u}, nodes, h, root_out, st, what);
 }
 
 extern "C" int zntt_probe_blake3(double* per_second) {
@@ -291,40 +280,26 @@ extern "C" int zntt_fri_fold_commit(int field, const uint64_t* d_layer, uint32_t
   cudaStream_t st = stream ? (cudaStream_t)stream : c.stream;
   uint4* nodes = reinterpret_cast<uint4*>(d_nodes);
   const uint32_t stride = log_table - log_n;
-  cudaError_t ce = cudaSuccess;
+  const char* what = "fri fold and commitment";
   if (small) {
     const uint64_t* tab = nullptr;
     uint64_t hv = 0, av = 0;
     int rc = small_fold_params(field, log_table, alpha, &tab, &hv, &av);
     if (rc) return rc;
-    ce = cudaMemsetAsync(nodes, 0, 32, st);
-    if (ce == cudaSuccess) {
-      if (field == kGoldilocksField)
-        ce = build_tree(SmallFoldLeafSource<Goldilocks>{d_layer, d_out, tab, h, stride, 8u, hv, av}, nodes, h, st);
-      else
-        ce = build_tree(SmallFoldLeafSource<BabyBear>{d_layer, d_out, tab, h, stride, 4u, hv, av}, nodes, h, st);
-    }
-  } else {
-    const void* tab = nullptr;
-    fe_pair av;
-    int rc = wide_fold_params(field, log_table, alpha, &tab, reinterpret_cast<uint64_t*>(&av));
-    if (rc) return rc;
-    const uint4* prev = reinterpret_cast<const uint4*>(d_layer);
-    uint4* next = reinterpret_cast<uint4*>(d_out);
-    const uint4* t4 = reinterpret_cast<const uint4*>(tab);
-    ce = cudaMemsetAsync(nodes, 0, 32, st);
-    if (ce == cudaSuccess) {
-      if (field == kBn254Fr)
-        ce = build_tree(WideFoldLeafSource<Bn254Fr>{prev, next, t4, h, stride, av}, nodes, h, st);
-      else
-        ce = build_tree(WideFoldLeafSource<Bls12381Fr>{prev, next, t4, h, stride, av}, nodes, h, st);
-    }
+    if (field == kGoldilocksField)
+      return commit_tree(SmallFoldLeafSource<Goldilocks>{d_layer, d_out, tab, h, stride, 8u, hv, av}, nodes, h, root_out,
+                         st, what);
+    return commit_tree(SmallFoldLeafSource<BabyBear>{d_layer, d_out, tab, h, stride, 4u, hv, av}, nodes, h, root_out, st,
+                       what);
   }
-  if (ce == cudaSuccess && root_out) {
-    ce = cudaMemcpyAsync(root_out, d_nodes + 32, 32, cudaMemcpyDeviceToHost, st);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-  }
-  if (ce != cudaSuccess) return cuda_fail(ce, "fri fold and commitment");
-  return ZNTT_OK;
+  const void* tab = nullptr;
+  fe_pair av;
+  int rc = wide_fold_params(field, log_table, alpha, &tab, reinterpret_cast<uint64_t*>(&av));
+  if (rc) return rc;
+  const uint4* prev = reinterpret_cast<const uint4*>(d_layer);
+  uint4* next = reinterpret_cast<uint4*>(d_out);
+  const uint4* t4 = reinterpret_cast<const uint4*>(tab);
+  if (field == kBn254Fr)
+    return commit_tree(WideFoldLeafSource<Bn254Fr>{prev, next, t4, h, stride, av}, nodes, h, root_out, st, what);
+  return commit_tree(WideFoldLeafSource<Bls12381Fr>{prev, next, t4, h, stride, av}, nodes, h, root_out, st, what);
 }
-

@@ -73,12 +73,13 @@ using namespace zntt;
 namespace {
 
 template <int FIELD>
-cudaError_t commit_rows_typed(const uint64_t* const* cols, uint32_t m, uint64_t n, uint4* nodes, cudaStream_t st) {
+int commit_rows_typed(const uint64_t* const* cols, uint32_t m, uint64_t n, uint4* nodes, uint8_t* root_out,
+                      cudaStream_t st) {
   RowLeafSource<FIELD> src;
   for (uint32_t c = 0; c < m; c++) src.col[c] = cols[c];
   for (uint32_t c = m; c < RowLeafSource<FIELD>::kMaxCols; c++) src.col[c] = nullptr;
   src.m = m;
-  return build_tree(src, nodes, n, st);
+  return commit_tree(src, nodes, n, root_out, st, "row commitment");
 }
 
 }  // namespace
@@ -110,19 +111,10 @@ extern "C" int zntt_merkle_commit_rows(int field, const uint64_t* const* d_colum
   std::lock_guard<std::recursive_mutex> lock(c.mu);
   cudaStream_t st = stream ? (cudaStream_t)stream : c.stream;
   uint4* nodes = reinterpret_cast<uint4*>(d_nodes);
-  cudaError_t ce = cudaMemsetAsync(nodes, 0, 32, st);
-  if (ce == cudaSuccess) {
-    switch (field) {
-      case kBn254Fr: ce = commit_rows_typed<kBn254Fr>(d_columns, num_columns, n, nodes, st); break;
-      case kBls12381Fr: ce = commit_rows_typed<kBls12381Fr>(d_columns, num_columns, n, nodes, st); break;
-      case kGoldilocksField: ce = commit_rows_typed<kGoldilocksField>(d_columns, num_columns, n, nodes, st); break;
-      default: ce = commit_rows_typed<kBabyBearField>(d_columns, num_columns, n, nodes, st);
-    }
+  switch (field) {
+    case kBn254Fr: return commit_rows_typed<kBn254Fr>(d_columns, num_columns, n, nodes, root_out, st);
+    case kBls12381Fr: return commit_rows_typed<kBls12381Fr>(d_columns, num_columns, n, nodes, root_out, st);
+    case kGoldilocksField: return commit_rows_typed<kGoldilocksField>(d_columns, num_columns, n, nodes, root_out, st);
+    default: return commit_rows_typed<kBabyBearField>(d_columns, num_columns, n, nodes, root_out, st);
   }
-  if (ce == cudaSuccess && root_out) {
-    ce = cudaMemcpyAsync(root_out, d_nodes + 32, 32, cudaMemcpyDeviceToHost, st);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-  }
-  if (ce != cudaSuccess) return cuda_fail(ce, "row commitment");
-  return ZNTT_OK;
 }

@@ -153,6 +153,54 @@ struct PoolBuf {
 };
 
 // ---------------------------------------------------------------------------
+// commitment roots
+// ---------------------------------------------------------------------------
+
+int root_wait_begin(uint64_t subtrees, RootWait* out) {
+  Context& c = ctx();
+  // subtrees / 16 counters for the first level of sixteens, then a sixteenth of
+  // those, ..., and one for each level of fewer than sixteen.
+  const size_t words = subtrees / 15 + 16;
+  if (words > c.tickets_words) {
+    if (c.tickets) cudaFree(c.tickets);
+    c.tickets = nullptr;
+    c.tickets_words = 0;
+    const size_t get = std::max<size_t>(words, 4096);
+    ZCHECK(cudaMalloc((void**)&c.tickets, get * 4), "tree counters");
+    cudaError_t e = cudaMemsetAsync(c.tickets, 0, get * 4, c.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
+    if (e != cudaSuccess) return cuda_fail(e, "tree counters");
+    c.tickets_words = get;
+  }
+  if (!c.root_host) {
+    ZCHECK(cudaHostAlloc(&c.root_host, 64, cudaHostAllocDefault), "pinned root");
+    std::memset(c.root_host, 0, 64);
+    c.root_seq = 0;
+  }
+  out->tickets = c.tickets;
+  out->root = c.root_host;
+  out->seq = reinterpret_cast<volatile uint32_t*>(static_cast<char*>(c.root_host) + 32);
+  out->value = ++c.root_seq;
+  return ZNTT_OK;
+}
+
+int root_wait(const RootWait& w, cudaStream_t st, uint8_t* root_out, const char* what) {
+  // The root arrives while the kernel's launch is still being retired: reading it
+  // as it lands saves a copy and most of a stream synchronisation per round.  A
+  // launch that failed never writes it, which the stream's status tells.
+  for (uint32_t spin = 1; *w.seq != w.value; spin++) {
+    if (spin % 4096) continue;
+    const cudaError_t e = cudaStreamQuery(st);
+    if (e == cudaErrorNotReady) continue;
+    if (e != cudaSuccess) return cuda_fail(e, what);
+    if (*w.seq != w.value) return set_error(ZNTT_ERR_DEVICE, std::string(what) + ": no root");
+  }
+  __atomic_thread_fence(__ATOMIC_ACQUIRE);
+  std::memcpy(root_out, w.root, 32);
+  return ZNTT_OK;
+}
+
+// ---------------------------------------------------------------------------
 // pass planning
 // ---------------------------------------------------------------------------
 
@@ -623,6 +671,11 @@ int zntt_shutdown(void) {
   fri_shutdown();
   free_coset_tabs();
   c.regs.clear();
+  if (c.tickets) cudaFree(c.tickets);
+  c.tickets = nullptr;
+  c.tickets_words = 0;
+  if (c.root_host) cudaFreeHost(c.root_host);
+  c.root_host = nullptr;
   c.pool.release_all();
   for (cudaStream_t& p : c.pipe)
     if (p) {
