@@ -97,7 +97,7 @@ static void launch_pass_full(bool ext, const PassParams& pp, dim3 grid, cudaStre
   const int smem = shape_smem_bytes(SH);
   if (ext)
     launch_pass_kernel(ntt_pass_kernel<F, S.log_tile, T, S.min_blocks, true, FULL, true>, T, smem, pp, grid, st);
-  else if (pp.scale || F::kScaleCompiled)
+  else if (pp.scale)
     launch_pass_kernel(ntt_pass_kernel<F, S.log_tile, T, S.min_blocks, false, FULL, true>, T, smem, pp, grid, st);
   else
     launch_pass_kernel(ntt_pass_kernel<F, S.log_tile, T, S.min_blocks, false, FULL, false>, T, smem, pp, grid, st);

@@ -11,10 +11,13 @@
 // ones where a Montgomery product costs 136 full ones: 214 multiply-pipe slots
 // of a 32-bit multiply-add against 272.  The transforms are bound by that pipe.
 //
-// Which x: any value below 2^256.  The quotient estimate drops the columns of
-// x q below word 6, worth less than 6 * 2^224 + 2^198, so with
-// q > w 2^256 / p - 1 it is above x w / p - x / 2^256 - 1 - 2^-29 and
-//   0 <= result < (1 + x / 2^256 + 2^-29) p.
+// Which x: any value below 2^256 / 1.03 (lazy fields; below 2p for the others).  The
+// quotient estimate drops the columns of x q below 6, worth less than 2^227, and
+// takes column 6's products x_i q_(6-i) from the 16 top bits of x_i and the 8 top
+// bits of q_(6-i), each low by less than (2^24 + 2^16) 2^224: in all less than
+// 0.0274 2^256, so with q > w 2^256 / p - 1 it is above
+// x w / p - x / 2^256 - 1 - 0.0274 and
+//   0 <= result < (1.0274 + x / 2^256) p.
 //
 // The factor is the plain value w, not its Montgomery form: x in Montgomery
 // form times w is the product in Montgomery form.  Both parts come out of one
@@ -171,41 +174,66 @@ __device__ __forceinline__ fe fe_add_raw(const fe& a, const fe& b) {
   return r;
 }
 
-// Words 8..15 of x * b, from the columns 6..14 of the product (above).  Even
-// columns accumulate in e (word 6 on), odd ones in o (word 7 on).
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+// c + the products of a's two 16-bit halves with b's two low (high) bytes.
+__device__ __forceinline__ uint32_t dp2a_lo(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t r;
+  asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+  return r;
+}
+__device__ __forceinline__ uint32_t dp2a_hi(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t r;
+  asm("dp2a.hi.u32.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+  return r;
+}
+
+// Words 8..15 of x * b, from the columns 7..14 of the product and an estimate of
+// column 6 (above).  Even columns accumulate in e (word 8 on), odd ones in o (word
+// 7 on).  The estimate, 35 bits at word 7, starts them, one word each: the first
+// product of a column takes a word more without a carry, but not two.
 __device__ __forceinline__ fe mul_high(const fe& x, const fe& b) {
-  uint32_t e6 = 0, e7 = 0, e8 = 0, e9 = 0, e10, e11 = 0, e12, e13 = 0, e14, e15 = 0;
-  uint32_t o7 = 0, o8 = 0, o9, o10 = 0, o11, o12 = 0, o13, o14 = 0, o15;
-  mad1(e6, e7, b.v[6], x.v[0]);
+  // Column 6: the 16 top bits of x_i times the 8 top bits of b_(6-i).
+  const uint32_t x01 = prmt(x.v[0], x.v[1], 0x7632), x23 = prmt(x.v[2], x.v[3], 0x7632),
+                 x45 = prmt(x.v[4], x.v[5], 0x7632), x6 = x.v[6] >> 16;
+  const uint32_t b6543 = prmt(prmt(b.v[6], b.v[5], 0x0073), prmt(b.v[4], b.v[3], 0x0073), 0x5410),
+                 b210 = prmt(prmt(b.v[2], b.v[1], 0x0073), b.v[0], 0x0710);
+  uint32_t c6 = dp2a_lo(x01, b6543, 0);
+  c6 = dp2a_hi(x23, b6543, c6);
+  c6 = dp2a_lo(x45, b210, c6);
+  c6 = dp2a_hi(x6, b210, c6);
+  uint32_t e8 = c6 >> 24, e9 = 0, e10 = 0, e11 = 0, e12, e13 = 0, e14, e15 = 0;
+  uint32_t o7 = c6 << 8, o8 = 0, o9, o10 = 0, o11, o12 = 0, o13, o14 = 0, o15;
   mad1(o7, o8, b.v[7], x.v[0]);
-  mad2(e6, e7, e8, e9, b.v[5], b.v[7], x.v[1]);
+  mad1(e8, e9, b.v[7], x.v[1]);
   mad1c(o7, o8, o9, b.v[6], x.v[1]);
-  mad2c(e6, e7, e8, e9, e10, b.v[4], b.v[6], x.v[2]);
+  mad1c(e8, e9, e10, b.v[6], x.v[2]);
   mad2(o7, o8, o9, o10, b.v[5], b.v[7], x.v[2]);
-  mad3(e6, e7, e8, e9, e10, e11, b.v[3], b.v[5], b.v[7], x.v[3]);
+  mad2(e8, e9, e10, e11, b.v[5], b.v[7], x.v[3]);
   mad2c(o7, o8, o9, o10, o11, b.v[4], b.v[6], x.v[3]);
-  mad3c(e6, e7, e8, e9, e10, e11, e12, b.v[2], b.v[4], b.v[6], x.v[4]);
+  mad2c(e8, e9, e10, e11, e12, b.v[4], b.v[6], x.v[4]);
   mad3(o7, o8, o9, o10, o11, o12, b.v[3], b.v[5], b.v[7], x.v[4]);
-  mad4(e6, e7, e8, e9, e10, e11, e12, e13, b.v[1], b.v[3], b.v[5], b.v[7], x.v[5]);
+  mad3(e8, e9, e10, e11, e12, e13, b.v[3], b.v[5], b.v[7], x.v[5]);
   mad3c(o7, o8, o9, o10, o11, o12, o13, b.v[2], b.v[4], b.v[6], x.v[5]);
-  mad4c(e6, e7, e8, e9, e10, e11, e12, e13, e14, b.v[0], b.v[2], b.v[4], b.v[6], x.v[6]);
+  mad3c(e8, e9, e10, e11, e12, e13, e14, b.v[2], b.v[4], b.v[6], x.v[6]);
   mad4(o7, o8, o9, o10, o11, o12, o13, o14, b.v[1], b.v[3], b.v[5], b.v[7], x.v[6]);
   mad4(e8, e9, e10, e11, e12, e13, e14, e15, b.v[1], b.v[3], b.v[5], b.v[7], x.v[7]);
   mad4c(o7, o8, o9, o10, o11, o12, o13, o14, o15, b.v[0], b.v[2], b.v[4], b.v[6], x.v[7]);
   fe r;
-  [[maybe_unused]] uint32_t w7;  // word 7 of the sum, for its carry
-  asm("add.cc.u32  %0, %9, %18;\n\t"
-      "addc.cc.u32 %1, %10, %19;\n\t"
-      "addc.cc.u32 %2, %11, %20;\n\t"
-      "addc.cc.u32 %3, %12, %21;\n\t"
-      "addc.cc.u32 %4, %13, %22;\n\t"
-      "addc.cc.u32 %5, %14, %23;\n\t"
-      "addc.cc.u32 %6, %15, %24;\n\t"
-      "addc.cc.u32 %7, %16, %25;\n\t"
-      "addc.u32    %8, %17, %26;"
-      : "=r"(w7), "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]),
+  asm("add.cc.u32  %0, %8, %16;\n\t"
+      "addc.cc.u32 %1, %9, %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, %23;"
+      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]),
         "=r"(r.v[7])
-      : "r"(e7), "r"(e8), "r"(e9), "r"(e10), "r"(e11), "r"(e12), "r"(e13), "r"(e14), "r"(e15), "r"(o7), "r"(o8),
+      : "r"(e8), "r"(e9), "r"(e10), "r"(e11), "r"(e12), "r"(e13), "r"(e14), "r"(e15), "r"(o8),
         "r"(o9), "r"(o10), "r"(o11), "r"(o12), "r"(o13), "r"(o14), "r"(o15));
   return r;
 }
@@ -276,8 +304,8 @@ __device__ __forceinline__ void mul_low_add_hi6(low_acc& s, const fe& x, const f
   s.o[7] += b.v[0] * x.v[5];
 }
 
-// x * w mod p up to a multiple of p, below (1 + x / 2^256 + 2^-29) p, for the
-// fixed factor (w, q).
+// x * w mod p up to a multiple of p, below (1.0274 + x / 2^256) p, for the fixed
+// factor (w, q).
 //
 // BLS12-381-Fr's low limbs make 28 of the 64 slots of quotient * p shifts and
 // adds: p = h 2^64 + 2^64 - 2^32 + 1 with h = floor(p / 2^64), so -t p is
@@ -374,15 +402,15 @@ static __device__ const __align__(16) Multiples kBnMultiples = make_multiples<Bn
 
 // The ranges of the butterflies, u, v -> u + t, u - t with t = w v.
 //
-// Lazy fields (BN254-Fr: 2^256 = 5.29 p).  v may be any value below 2^256 and
-// t stays below 2 p, so only u needs a bound, and two stages in a row need it
-// once: from u < 1.07 p the first stage's results are below 3.07 p and, as u of
-// the second stage, lead to results below 5.07 p < 2^256.  fe_weak brings a
+// Lazy fields (BN254-Fr: 2^256 = 5.29 p).  v may be any value below 5.07 p, for
+// which t stays below 1.986 p, so only u needs a bound, and two stages in a row
+// need it once: from u < 1.07 p the first stage's results are below 3.07 p and,
+// as u of the second stage, lead to results below 5.07 p < 2^256.  fe_weak brings a
 // stored value (or a v whose factor is one) below 1.07 p: k = floor of its top
 // byte over 49 (p is 48.39 of those units) is at most x / p and at least
 // x / p - 1.07.
-// Other fields (BLS12-381-Fr: 2^256 = 2.21 p) keep values below 2 p: u and t are
-// reduced to [0, p) before each butterfly.
+// Other fields (BLS12-381-Fr: 2^256 = 2.21 p) keep values below 2 p, for which t is
+// below 1.934 p: u and t are reduced to [0, p) before each butterfly.
 template <class F>
 __device__ __forceinline__ fe fe_weak(const fe& x) {
   if constexpr (F::kLazy) {
