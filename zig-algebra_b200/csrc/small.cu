@@ -46,6 +46,7 @@ struct SmallHost {
     return r1;
   }
   uint64_t inv(uint64_t a) const { return pow(a, p - 2); }  // p prime; inv(0) = 0
+  uint64_t half() const { return (p >> 1) + 1; }             // 1/2
   uint64_t to_tw(uint64_t w) const { return mul(w % p, r); }
 };
 
@@ -459,6 +460,7 @@ struct SmallTable {
   bool tw0_one = true;
   bool foreign = false;
   uint64_t last_use = 0;
+  uint64_t n_inv = 0;         // 1/n, canonical
 };
 
 struct SmallRegistration {
@@ -544,6 +546,7 @@ int small_acquire(int field, uint32_t log_n, uint64_t root, SmallTable** out) {
   e->field = field;
   e->log_n = log_n;
   e->root = root;
+  e->n_inv = H.inv(((uint64_t)1 << log_n) % H.p);
   e->bytes = small_entries(log_n) * 8;
   small_evict(e->bytes);
   cudaError_t ce = cudaMalloc((void**)&e->d_table, e->bytes);
@@ -594,6 +597,7 @@ int small_upload_foreign(int field, uint32_t log_n, const zntt_stage* stages, Sm
   e->field = field;
   e->log_n = log_n;
   e->foreign = true;
+  e->n_inv = small_host(field).inv(((uint64_t)1 << log_n) % small_host(field).p);
   e->bytes = small_entries(log_n) * 8;
   cudaError_t ce = cudaMalloc((void**)&e->d_table, e->bytes);
   if (ce != cudaSuccess) {
@@ -729,7 +733,8 @@ int small_transform_host(const SmallTable* t, uint64_t* data, bool inverse, bool
   return rc;
 }
 
-uint64_t n_inverse_tw(const SmallHost& H, uint32_t log_n) { return H.to_tw(H.inv(((uint64_t)1 << log_n) % H.p)); }
+// The inverse's scale factor, in twiddle form.
+uint64_t n_inverse_tw(const SmallTable* t) { return small_host(t->field).to_tw(t->n_inv); }
 
 int check_small_shape(size_t len, size_t log_n) {
   if (log_n >= 64) return set_error(ZNTT_ERR_LOG_TOO_LARGE, "log_n >= 64");
@@ -819,7 +824,7 @@ int small_ntt_root(int field, uint64_t* data, size_t len, size_t log_n, const ui
   SmallTable* t = nullptr;
   rc = small_acquire(field, (uint32_t)log_n, r, &t);
   if (rc) return rc;
-  rc = small_transform_host(t, data, false, inverse, n_inverse_tw(H, (uint32_t)log_n));
+  rc = small_transform_host(t, data, false, inverse, n_inverse_tw(t));
   small_release(t);
   return rc;
 }
@@ -926,7 +931,7 @@ int small_ntt_with_twiddles(int field, uint64_t* data, size_t len, size_t log_n,
     if (rc) return rc;
     foreign = true;
   }
-  rc = small_transform_host(t, data, inverse, inverse, n_inverse_tw(H, (uint32_t)log_n));
+  rc = small_transform_host(t, data, inverse, inverse, n_inverse_tw(t));
   if (foreign) small_release(t);
   return rc;
 }
@@ -962,7 +967,7 @@ int small_ntt_device(const zntt_twiddles* tw, const uint64_t* d_src, uint64_t* d
   const SmallTable* t = reinterpret_cast<const SmallTable*>(tw);
   const SmallHost& H = small_host(t->field);
   const bool inverse = mode == ZNTT_INVERSE;
-  const uint64_t ninv = n_inverse_tw(H, t->log_n);
+  const uint64_t ninv = n_inverse_tw(t);
   cudaStream_t st = stream ? (cudaStream_t)stream : c.stream;
   const bool need_scratch = d_src == d_dst && small_plan(t->log_n, inverse || t->tw0_one).passes.size() > 1;
   if (need_scratch && !d_scratch) {
@@ -1032,7 +1037,7 @@ int small_fold_params(int field, uint32_t log_table, const uint64_t* alpha, cons
   std::lock_guard<std::recursive_mutex> lock(c.mu);
   auto& tabs = small_fold_tables();
   const auto key = std::make_pair(field, log_table);
-  const uint64_t half_inv = H.inv(2);
+  const uint64_t half_inv = H.half();
   auto it = tabs.find(key);
   if (it != tabs.end()) {
     *tab_out = it->second;
@@ -1161,7 +1166,7 @@ int small_coset_lde_many(const zntt_twiddles* tw_in, const zntt_twiddles* tw_out
     // first power table); else the inverse scales by n^-1 and a launch of its own
     // by shift^i.
     const bool fused = small_plan(ti->log_n, true).tiles;
-    const uint64_t n_inv = H.inv(n_in % H.p);
+    const uint64_t n_inv = ti->n_inv;
     cudaError_t ce = launch_small_power_tables(ti->field, shift[0], fused ? n_inv : 1, (uint64_t*)d_pw, st);
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(tabs, h.data(), tab_bytes, cudaMemcpyHostToDevice, st);
     if (ce == cudaSuccess) {
@@ -1201,7 +1206,7 @@ int small_coset_lde_many(const zntt_twiddles* tw_in, const zntt_twiddles* tw_out
   cudaError_t ce = launch_small_power_tables(ti->field, shift[0], 1, (uint64_t*)d_pw, st);
   for (uint32_t k = 0; k < m && ce == cudaSuccess && rc == ZNTT_OK; k++) {
     uint64_t* out = d_out[k];
-    rc = small_run(ti, d_evals[k], out, nullptr, true, true, n_inverse_tw(H, ti->log_n), st);  // out of place
+    rc = small_run(ti, d_evals[k], out, nullptr, true, true, n_inverse_tw(ti), st);  // out of place
     if (rc) break;
     if (ti->field == kGoldilocksField)
       small_coset_scale_kernel<Goldilocks><<<grid_for(n_in), 256, 0, st>>>((const uint64_t*)d_pw, out, n_in);
@@ -1300,7 +1305,7 @@ int small_poly_mul(int field, const uint64_t* a, size_t a_len, const uint64_t* b
     ce = cudaGetLastError();
     if (ce != cudaSuccess) rc = cuda_fail(ce, "pointwise product");
   }
-  if (!rc) rc = small_run(t, A, B, S, true, true, n_inverse_tw(H, L), st);  // coefficients into B
+  if (!rc) rc = small_run(t, A, B, S, true, true, n_inverse_tw(t), st);  // coefficients into B
   if (!rc) {
     ce = cudaMemcpyAsync(out, B, lo * 8, cudaMemcpyDeviceToHost, st);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
@@ -1360,7 +1365,7 @@ int small_ntt_columns(const zntt_twiddles* tw, const uint64_t* const* d_src, uin
   ce = cudaMemcpyAsync(tabs, h.data(), tab_bytes, cudaMemcpyHostToDevice, st);
   if (ce == cudaSuccess)
     rc = small_run_cols(t, m, static_cast<const uint64_t* const*>(tabs), static_cast<uint64_t* const*>(tabs) + m,
-                        (uint32_t)n, inverse, inverse, inverse ? n_inverse_tw(H, t->log_n) : 0, st);
+                        (uint32_t)n, inverse, inverse, inverse ? n_inverse_tw(t) : 0, st);
   cudaError_t ce2 = cudaStreamSynchronize(st);
   pool_put(tabs, tab_bytes);
   if (rc) return rc;
