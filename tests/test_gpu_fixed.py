@@ -120,3 +120,32 @@ def test_captured_transforms_replay(z, log_n):
             graph.replay()
             stream.synchronize()
             assert torch.equal(mid, want) and torch.equal(dst, src)
+
+
+@pytest.mark.parametrize("log_n", [8, 9, 11])
+def test_in_place_without_scratch_can_be_captured(z, log_n):
+    """Up to the untuned plan's tile (2^11; 2^12 for the small fields) an in-place transform needs
+    no scratch: it neither waits nor allocates, so a caller's graph can hold it."""
+    import torch
+    z.tune_clear()
+    stream = torch.cuda.Stream()
+    for F, L in ((z.BN254_FR, log_n), (z.BLS12_381_FR, log_n), (z.GOLDILOCKS, log_n + 1), (z.BABYBEAR, log_n + 1)):
+        words = F.limbs << L
+        with z.DeviceTwiddles(F, L, z.primitiveRootOfUnity(F, L)) as tw, torch.cuda.stream(stream):
+            data = torch.zeros(words, dtype=torch.int64, device="cuda")
+            if F.limbs == 4:
+                z.random_elements(F, L, data.data_ptr(), 1 << L, stream=stream.cuda_stream)
+            else:
+                data += torch.randint(0, F.modulus if F.name == "babybear" else 1 << 62, (words,), device="cuda")
+            orig, want = data.clone(), torch.zeros_like(data)
+            z.ntt_device(tw, data.data_ptr(), want.data_ptr(), z.FORWARD, stream=stream.cuda_stream)
+            stream.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                z.ntt_device(tw, data.data_ptr(), data.data_ptr(), z.FORWARD, stream=stream.cuda_stream)
+            graph.replay()
+            stream.synchronize()
+            assert torch.equal(data, want), F.name
+            z.ntt_device(tw, data.data_ptr(), data.data_ptr(), z.INVERSE, stream=stream.cuda_stream)
+            stream.synchronize()
+            assert torch.equal(data, orig), F.name

@@ -423,11 +423,12 @@ struct SmallPlan {
 // on whole tiles, with passes of six to ten stages: a pass of ten exchanges
 // twice but saves a sweep (2^20 Goldilocks forward 0.0327 ms as 10 + 10 stages,
 // 0.0368 as 7 + 7 + 6; both are faster than this file's own passes at every size
-// from 2^12, 0.0143 ms against 0.0205 there, B200).
-SmallPlan small_plan(uint32_t log_n, bool unit0) {
+// from 2^12, 0.0143 ms against 0.0205 there, B200).  `one_pass`: in place without
+// scratch, where one pass keeps the call asynchronous up to 2^12.
+SmallPlan small_plan(uint32_t log_n, bool unit0, bool one_pass = false) {
   SmallPlan plan;
   if (log_n == 0) return plan;
-  plan.tiles = unit0 && log_n >= kTileLog;
+  plan.tiles = unit0 && log_n >= (uint32_t)kTileLog + one_pass;
   const uint32_t lt = plan.tiles ? kTileLog : kSmallLogTile, kmax = plan.tiles ? kTileKmax : kSmallKmax;
   if (log_n <= lt && !plan.tiles) {
     plan.passes.push_back({0, log_n, 0});
@@ -677,7 +678,7 @@ int small_run_cols(const SmallTable* t, uint32_t m, const uint64_t* const* srcs,
 
 int small_run(const SmallTable* t, const uint64_t* src, uint64_t* dst, uint64_t* scratch, bool inverse, bool scale,
               uint64_t scale_tw, cudaStream_t st) {
-  const SmallPlan plan = small_plan(t->log_n, inverse || t->tw0_one);
+  const SmallPlan plan = small_plan(t->log_n, inverse || t->tw0_one, src == dst && !scratch);
   const size_t np = plan.passes.size();
   if (np == 0) {  // one element: a copy (the 1/n scale is by one)
     if (src != dst) {
@@ -969,7 +970,7 @@ int small_ntt_device(const zntt_twiddles* tw, const uint64_t* d_src, uint64_t* d
   const bool inverse = mode == ZNTT_INVERSE;
   const uint64_t ninv = n_inverse_tw(t);
   cudaStream_t st = stream ? (cudaStream_t)stream : c.stream;
-  const bool need_scratch = d_src == d_dst && small_plan(t->log_n, inverse || t->tw0_one).passes.size() > 1;
+  const bool need_scratch = d_src == d_dst && small_plan(t->log_n, inverse || t->tw0_one, !d_scratch).passes.size() > 1;
   if (need_scratch && !d_scratch) {
     const size_t bytes = ((size_t)8) << t->log_n;
     void* s = nullptr;
