@@ -180,8 +180,12 @@ __global__ void blake3_probe_kernel(uint32_t* sink, uint32_t iters, uint32_t one
 
 using namespace zntt;
 
-extern "C" int zntt_fri_commit_layer(int field, const uint64_t* d_layer, uint32_t log_n, uint8_t* d_nodes,
-                                     uint8_t* root_out, void* stream) {
+namespace zntt {
+
+// zntt_fri_commit_layer.  `settle`: with root_out, also wait until the stream has
+// retired the work (the commit phase's rounds need the root only).
+int fri_commit_layer(int field, const uint64_t* d_layer, uint32_t log_n, uint8_t* d_nodes, uint8_t* root_out,
+                     void* stream, bool settle) {
   clear_error();
   const bool small = is_small_field(field);
   if (!small && field != kBn254Fr && field != kBls12381Fr)
@@ -202,9 +206,16 @@ extern "C" int zntt_fri_commit_layer(int field, const uint64_t* d_layer, uint32_
   uint4* nodes = reinterpret_cast<uint4*>(d_nodes);
   const uint4* wide = reinterpret_cast<const uint4*>(d_layer);
   const char* what = "fri layer commitment";
-  if (field == kBn254Fr) return commit_tree(WideLeafSource<Bn254Fr>{wide, h}, nodes, h, root_out, st, what);
-  if (field == kBls12381Fr) return commit_tree(WideLeafSource<Bls12381Fr>{wide, h}, nodes, h, root_out, st, what);
-  return commit_tree(SmallLeafSource{d_layer, h, field == kGoldilocksField ? 8u : 4u}, nodes, h, root_out, st, what);
+  if (field == kBn254Fr) return commit_tree(WideLeafSource<Bn254Fr>{wide, h}, nodes, h, root_out, st, settle, what);
+  if (field == kBls12381Fr) return commit_tree(WideLeafSource<Bls12381Fr>{wide, h}, nodes, h, root_out, st, settle, what);
+  return commit_tree(SmallLeafSource{d_layer, h, field == kGoldilocksField ? 8u : 4u}, nodes, h, root_out, st, settle, what);
+}
+
+}  // namespace zntt
+
+extern "C" int zntt_fri_commit_layer(int field, const uint64_t* d_layer, uint32_t log_n, uint8_t* d_nodes,
+                                     uint8_t* root_out, void* stream) {
+  return fri_commit_layer(field, d_layer, log_n, d_nodes, root_out, stream, true);
 }
 
 extern "C" int zntt_probe_blake3(double* per_second) {
@@ -240,9 +251,11 @@ extern "C" int zntt_probe_blake3(double* per_second) {
   return ZNTT_OK;
 }
 
-extern "C" int zntt_fri_fold_commit(int field, const uint64_t* d_layer, uint32_t log_n, const uint64_t alpha[4],
-                                    uint64_t* d_out, uint32_t log_table, uint8_t* d_nodes, uint8_t* root_out,
-                                    void* stream) {
+namespace zntt {
+
+// zntt_fri_fold_commit, with `settle` as above.
+int fri_fold_commit(int field, const uint64_t* d_layer, uint32_t log_n, const uint64_t alpha[4], uint64_t* d_out,
+                    uint32_t log_table, uint8_t* d_nodes, uint8_t* root_out, void* stream, bool settle) {
   clear_error();
   const bool small = is_small_field(field);
   if (!small && field != kBn254Fr && field != kBls12381Fr)
@@ -288,9 +301,9 @@ extern "C" int zntt_fri_fold_commit(int field, const uint64_t* d_layer, uint32_t
     if (rc) return rc;
     if (field == kGoldilocksField)
       return commit_tree(SmallFoldLeafSource<Goldilocks>{d_layer, d_out, tab, h, stride, 8u, hv, av}, nodes, h, root_out,
-                         st, what);
+                         st, settle, what);
     return commit_tree(SmallFoldLeafSource<BabyBear>{d_layer, d_out, tab, h, stride, 4u, hv, av}, nodes, h, root_out, st,
-                       what);
+                       settle, what);
   }
   const void* tab = nullptr;
   fe_pair av;
@@ -300,6 +313,14 @@ extern "C" int zntt_fri_fold_commit(int field, const uint64_t* d_layer, uint32_t
   uint4* next = reinterpret_cast<uint4*>(d_out);
   const uint4* t4 = reinterpret_cast<const uint4*>(tab);
   if (field == kBn254Fr)
-    return commit_tree(WideFoldLeafSource<Bn254Fr>{prev, next, t4, h, stride, av}, nodes, h, root_out, st, what);
-  return commit_tree(WideFoldLeafSource<Bls12381Fr>{prev, next, t4, h, stride, av}, nodes, h, root_out, st, what);
+    return commit_tree(WideFoldLeafSource<Bn254Fr>{prev, next, t4, h, stride, av}, nodes, h, root_out, st, settle, what);
+  return commit_tree(WideFoldLeafSource<Bls12381Fr>{prev, next, t4, h, stride, av}, nodes, h, root_out, st, settle, what);
+}
+
+}  // namespace zntt
+
+extern "C" int zntt_fri_fold_commit(int field, const uint64_t* d_layer, uint32_t log_n, const uint64_t alpha[4],
+                                    uint64_t* d_out, uint32_t log_table, uint8_t* d_nodes, uint8_t* root_out,
+                                    void* stream) {
+  return fri_fold_commit(field, d_layer, log_n, alpha, d_out, log_table, d_nodes, root_out, stream, true);
 }

@@ -159,10 +159,10 @@ int zntt_fri_commit_phase(int field, uint32_t log_domain, uint32_t log_final, ui
     uint8_t* root = roots_out + 32 * (size_t)r;
     const uint32_t log_n = log_domain - r;
     if (r == 0)
-      rc = zntt_fri_commit_layer(field, d_layers[0], log_n, d_nodes[0], root, stream);  // waits for the root
+      rc = fri_commit_layer(field, d_layers[0], log_n, d_nodes[0], root, stream, false);  // waits for the root
     else
-      rc = zntt_fri_fold_commit(field, d_layers[r - 1], log_n + 1, alpha, d_layers[r], log_domain, d_nodes[r], root,
-                                stream);
+      rc = fri_fold_commit(field, d_layers[r - 1], log_n + 1, alpha, d_layers[r], log_domain, d_nodes[r], root, stream,
+                           false);
     if (rc) return rc;
     for (int k = 0; k < 4; k++) alpha[k] = 0;
     const int cs = challenge(user, r, root, alpha);

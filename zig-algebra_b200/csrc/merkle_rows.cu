@@ -79,7 +79,7 @@ int commit_rows_typed(const uint64_t* const* cols, uint32_t m, uint64_t n, uint4
   for (uint32_t c = 0; c < m; c++) src.col[c] = cols[c];
   for (uint32_t c = m; c < RowLeafSource<FIELD>::kMaxCols; c++) src.col[c] = nullptr;
   src.m = m;
-  return commit_tree(src, nodes, n, root_out, st, "row commitment");
+  return commit_tree(src, nodes, n, root_out, st, true, "row commitment");
 }
 
 }  // namespace

@@ -260,27 +260,23 @@ cudaError_t build_tree(const Src& src, uint4* nodes, uint64_t h, cudaStream_t st
   return ce;
 }
 
-// The same tree for a caller that waits for its root: one launch (after one for
-// leaves that run one per thread), which delivers the root itself.
-template <class Src>
-cudaError_t build_tree_root(const Src& src, uint4* nodes, uint64_t h, uint32_t* tickets, const RootOut& out,
-                            cudaStream_t st) {
-  if (h <= kThreads) {
-    small_tree_kernel<Src><<<1, kThreads, 0, st>>>(src, nodes, (uint32_t)h, out, 1u);
-    return cudaGetLastError();
+// Levels of at least this width get launches of their own, one per five levels:
+// with as many CTAs the fences and counts of tree_kernel cost more than launches
+// save.  A Goldilocks layer and its root, one launch against this line: 2^18 42.5
+// and 41 us, 2^20 72 and 67, 2^24 560 and 516; below it one launch is the faster
+// (2^16 33.9 us, 43.5 in launches; lines at 2^19 and 2^21 are no faster; B200).
+constexpr uint64_t kOwnLaunchWidth = (uint64_t)1 << 17;
+
+// tree_kernel over the level of width w, made by the launch before it on `st`.
+cudaError_t launch_node_tree(uint4* nodes, uint64_t w, uint32_t* tickets, const RootOut& out, cudaStream_t st) {
+  for (; w >= kOwnLaunchWidth; w >>= 1 + kSharedLevels) {
+    subtree_kernel<NodeSource, false><<<(unsigned)(w / (2 * kThreads)), kThreads, 0, st>>>(NodeSource{nodes, w},
+                                                                                           nodes, w, 1u);
+    const cudaError_t ce = cudaGetLastError();
+    if (ce != cudaSuccess) return ce;
   }
-  const unsigned grid = (unsigned)(h / (2 * kThreads));
-  if (!OneLeafPerThread<Src>::value) {
-    tree_kernel<Src, true><<<grid, kThreads, 0, st>>>(src, nodes, h, tickets, out, 1u);
-    return cudaGetLastError();
-  }
-  // Few leaves: small CTAs, so that they spread over the SMs.
-  const uint32_t threads = h <= 148 * 256 ? 64 : kThreads;
-  leaf_kernel<Src><<<(unsigned)std::min<uint64_t>(h / threads, 148 * 16), threads, 0, st>>>(src, nodes, h, 1u);
-  cudaError_t ce = cudaGetLastError();
-  if (ce != cudaSuccess) return ce;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = dim3((unsigned)(w / (2 * kThreads)));
   cfg.blockDim = dim3(kThreads);
   cfg.stream = st;
   cudaLaunchAttribute attr;
@@ -288,14 +284,40 @@ cudaError_t build_tree_root(const Src& src, uint4* nodes, uint64_t h, uint32_t* 
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, tree_kernel<NodeSource, false>, NodeSource{nodes, h}, nodes, h, tickets, out, 1u);
+  return cudaLaunchKernelEx(&cfg, tree_kernel<NodeSource, false>, NodeSource{nodes, w}, nodes, w, tickets, out, 1u);
+}
+
+// The same tree for a caller that waits for its root: one launch where it is not
+// wide (after one for leaves that run one per thread), which delivers the root.
+template <class Src>
+cudaError_t build_tree_root(const Src& src, uint4* nodes, uint64_t h, uint32_t* tickets, const RootOut& out,
+                            cudaStream_t st) {
+  if (h <= kThreads) {
+    small_tree_kernel<Src><<<1, kThreads, 0, st>>>(src, nodes, (uint32_t)h, out, 1u);
+    return cudaGetLastError();
+  }
+  if (OneLeafPerThread<Src>::value) {
+    // Few leaves: small CTAs, so that they spread over the SMs.
+    const uint32_t threads = h <= 148 * 256 ? 64 : kThreads;
+    leaf_kernel<Src><<<(unsigned)std::min<uint64_t>(h / threads, 148 * 16), threads, 0, st>>>(src, nodes, h, 1u);
+    const cudaError_t ce = cudaGetLastError();
+    return ce == cudaSuccess ? launch_node_tree(nodes, h, tickets, out, st) : ce;
+  }
+  const unsigned grid = (unsigned)(h / (2 * kThreads));
+  if (h >= kOwnLaunchWidth) {
+    subtree_kernel<Src, true><<<grid, kThreads, 0, st>>>(src, nodes, h, 1u);
+    const cudaError_t ce = cudaGetLastError();
+    return ce == cudaSuccess ? launch_node_tree(nodes, h >> (1 + kSharedLevels), tickets, out, st) : ce;
+  }
+  tree_kernel<Src, true><<<grid, kThreads, 0, st>>>(src, nodes, h, tickets, out, 1u);
+  return cudaGetLastError();
 }
 
 // A commitment over h leaves on `st`.  With root_out it returns once the root is
-// there (and with it every node); the work of the stream before it is then done
-// too.  Without, it only enqueues.
+// there (and with it every node), or with `settle` once the stream has retired
+// the work.  Without root_out it only enqueues.
 template <class Src>
-int commit_tree(const Src& src, uint4* nodes, uint64_t h, uint8_t* root_out, cudaStream_t st, const char* what) {
+int commit_tree(const Src& src, uint4* nodes, uint64_t h, uint8_t* root_out, cudaStream_t st, bool settle, const char* what) {
   if (!root_out) {
     cudaError_t ce = cudaMemsetAsync(nodes, 0, 32, st);  // node 0 is unused and zero
     if (ce == cudaSuccess) ce = build_tree(src, nodes, h, st);
@@ -307,7 +329,10 @@ int commit_tree(const Src& src, uint4* nodes, uint64_t h, uint8_t* root_out, cud
   const cudaError_t ce =
       build_tree_root(src, nodes, h, wait.tickets, RootOut{static_cast<uint4*>(wait.root), wait.seq, wait.value}, st);
   if (ce != cudaSuccess) return cuda_fail(ce, what);
-  return root_wait(wait, st, root_out, what);
+  rc = root_wait(wait, st, root_out, what);
+  if (rc || !settle) return rc;
+  const cudaError_t se = cudaStreamSynchronize(st);
+  return se == cudaSuccess ? ZNTT_OK : cuda_fail(se, what);
 }
 
 }  // namespace

@@ -43,6 +43,11 @@ int small_coset_lde_many(const zntt_twiddles* tw_in, const zntt_twiddles* tw_out
                          const uint64_t* const* d_evals, uint64_t* const* d_out, uint32_t m, void* stream);
 int small_coset_lde(const zntt_twiddles* tw_in, const zntt_twiddles* tw_out, const uint64_t* shift,
                     const uint64_t* d_evals, uint64_t* d_out, void* stream);
+// The commitments of the prover's rounds (fri_commit.cu).
+int fri_commit_layer(int field, const uint64_t* d_layer, uint32_t log_n, uint8_t* d_nodes, uint8_t* root_out,
+                     void* stream, bool settle);
+int fri_fold_commit(int field, const uint64_t* d_layer, uint32_t log_n, const uint64_t alpha[4], uint64_t* d_out,
+                    uint32_t log_table, uint8_t* d_nodes, uint8_t* root_out, void* stream, bool settle);
 void small_shutdown();
 // FRI fold tables of the 256-bit fields (fri.cu).
 void fri_shutdown();
