@@ -46,9 +46,12 @@ import threading
 import time
 
 ROOT = os.path.dirname(os.path.abspath(__file__))
-# Multiply-pipe issue slots per 8x32-bit CIOS field product: 2N^2 + N = 136
-# full 32x32->64 products, each two 32-bit IMAD slots (lo and hi).
-IMAD_PER_MODMUL = 272
+# Multiply-pipe issue slots of a field product by a factor known beforehand (a
+# twiddle with its quotient), as the transforms make them: full 32x32->64
+# products of two 32-bit IMAD slots each, low products and dot products of one.
+# BN254-Fr 92 full, 16 low, 4 dot; BLS12-381-Fr 79 full, 14 low, 4 dot (its low
+# limbs' share is shifts and adds).  A Montgomery product takes 272.
+IMAD_PER_MODMUL = {"bn254_fr": 204, "bls12_381_fr": 176}
 METRIC = "BN254-Fr NTT elems/s at 2^24"
 
 
@@ -366,12 +369,12 @@ def run_zntt(args, rank, world, local):
 
     # Roofline: the pass kernel is the only kernel in the timed region.
     imad = z.probe_imad()
-    peak_modmul = imad / IMAD_PER_MODMUL
+    peak_modmul = imad / IMAD_PER_MODMUL["bn254_fr"]
     modmuls = n / 2 * log_n
     achieved = modmuls / (ms_step * 1e-3)
     peaks, peaks_kind = measured_peaks()
     alg_bytes = 2 * n * 32
-    passes = __import__("math").ceil(log_n / 10) if log_n > 11 else 1
+    passes = 1 if log_n <= 8 else 2 if log_n <= 18 else -(-log_n // 9)
     traffic = read_traffic(log_n)
     tw.close()
     extra = {}
@@ -380,7 +383,7 @@ def run_zntt(args, rank, world, local):
     # closing barrier for longer than the process group's timeout.
     if not args.headline_only and world == 1:
         with torch.cuda.stream(stream):
-            extra["sizes"] = run_size_sweep(z, torch, stream, steps=10, warmup=3, peak_modmul=peak_modmul)
+            extra["sizes"] = run_size_sweep(z, torch, stream, steps=10, warmup=3, imad=imad)
             extra["batched"] = run_batched_config(z, torch, stream, steps=20, warmup=3)
             extra["coset_lde"] = run_lde_config(z, torch, stream, steps=5, warmup=2)
             extra["poly_mul"] = run_poly_config(z, torch, stream, steps=5, warmup=2,
@@ -415,7 +418,7 @@ def run_zntt(args, rank, world, local):
         "roofline": {"bound": "imad", "achieved": achieved, "peak": peak_modmul, "unit": "modmul/s",
                      "frac": achieved / peak_modmul, "traffic": traffic,
                      "peak_source": f"measured live: dependent mad.lo.u32 probe {imad:.4g} IMAD/s / "
-                                    f"{IMAD_PER_MODMUL} IMAD slots per 8x32-bit CIOS modmul",
+                                    f"{IMAD_PER_MODMUL['bn254_fr']} IMAD slots per modmul by a fixed factor",
                      "hbm": {"achieved": alg_bytes / (ms_step * 1e-3) / 1e9, "peak": peaks["hbm_gbs"],
                              "unit": "GB/s", "frac": alg_bytes / (ms_step * 1e-3) / 1e9 / peaks["hbm_gbs"],
                              "peak_source": f"MEASURED_PEAKS.json hbm_gbs ({peaks_kind})"}},
@@ -505,7 +508,7 @@ def time_region(torch, stream, fn, steps):
     return e0.elapsed_time(e1)
 
 
-def run_size_sweep(z, torch, stream, steps, warmup, peak_modmul, seed=66):
+def run_size_sweep(z, torch, stream, steps, warmup, imad, seed=66):
     """The single-transform configuration across sizes and directions: BN254-Fr 2^20, 2^22 and
     2^24, forward and inverse (nttWithTwiddles / inttWithTwiddles, libs/ntt/src/root.zig:148-212),
     and BLS12-381-Fr 2^24, with the tables resident.  Each entry: ms per transform, elements/s,
@@ -532,7 +535,7 @@ def run_size_sweep(z, torch, stream, steps, warmup, peak_modmul, seed=66):
                     hbm_gbs = 2 * n * 32 / (ms * 1e-3) / 1e9
                     out[f"{F.name} 2^{L} {name}"] = {
                         "ms": ms, "elements_per_s": n / (ms * 1e-3), "modmul_per_s": modmuls / (ms * 1e-3),
-                        "frac": modmuls / (ms * 1e-3) / peak_modmul, "hbm_gbs": hbm_gbs,
+                        "frac": modmuls / (ms * 1e-3) * IMAD_PER_MODMUL[F.name] / imad, "hbm_gbs": hbm_gbs,
                         "hbm_frac": hbm_gbs / hbm_peak}
         del x, y
     return out

@@ -54,10 +54,10 @@ struct PassShape {
 };
 // 2^11 and 2^10 tiles in CTAs of 256 threads (3 per SM), and the same 24 warps
 // per SM in smaller CTAs: 2^9 tiles in 128 threads (6 per SM) and 2^8 tiles in
-// 64 threads (12 per SM), where each barrier waits on fewer warps (2^24
-// BN254-Fr: 3.65 ms with 2^10 tiles, 3.49 ms with 2^9 or 2^8 tiles, B200).
-// The last shape trades a 72-register budget (a few spilled words) for 28
-// warps per SM: 2^22 and 2^24 BN254-Fr about 0.6% faster, BLS12-381-Fr slower.
+// 64 threads (12 per SM), where each barrier waits on fewer warps.  The last
+// shape trades a 72-register budget (a few spilled words) for 28 warps per SM.
+// 2^24 BN254-Fr in ms, B200: 2^10 tiles 2.88, 2^9 at 7 CTAs 2.71 (and at 8 CTAs,
+// 64 registers, 2.80: not compiled), 2^8 tiles 3.09.
 constexpr int kNumShapes = 5;
 // Behind the tunable shapes, two of one butterfly per thread (ntt_tile_radix2),
 // kRadix2Shape with 2^7-element tiles and the next with 2^8.
@@ -70,10 +70,9 @@ constexpr int kRadix2Shape = kNumShapes;
 // on the radix-4 passes are as fast or faster (63.5 / 63.6, 2^18 106 / 102).
 constexpr uint32_t kRadix2MaxLog = 16;
 // The shape of persistent launches (batches and the server's slices): the
-// 7-CTA 2^9 tile ran the mixed 520-transform batch 3.03 -> 2.94 ms and 64
-// coset extensions 2^18 -> 2^20 16.95 -> 16.74 ms (BLS12-381-Fr) and 15.81 ->
-// 15.45 ms (BN254-Fr) against the 6-CTA tile, and the 2^10 and 2^8 tiles
-// slower still (B200).
+// 7-CTA 2^9 tile runs the mixed 520-transform batch in 2.22 ms, the 2^11 tile in
+// 2.26, the 6-CTA 2^9 tile 2.27, the 2^10 tile 2.37, the 2^8 tile 2.42; 64 coset
+// extensions 2^18 -> 2^20 (BLS12-381-Fr) 11.9 / 11.9 / 12.1 / 12.6 / 13.0 (B200).
 constexpr int kBatchShape = 4;
 constexpr int kLogTile = 11;  // the largest tile of any shape
 constexpr int kDefaultShape = 0;
