@@ -160,7 +160,11 @@ struct TilePass {
     if (SCALE && pp.scale) {
       const uint4* f = pp.scale_tab;
       if (EXT && pp.scale != kScaleFixed) f += (pp.scale == kScaleElements ? 2ull : 4ull) * g;
-      if (EXT && pp.scale == kScaleElements) y = fe_mul<F>(fe_load_nc(f), x);
+      // Elements are the other transform's output: in a batch other CTAs of this launch
+      // wrote them (so they go through L2, as the tile's data does), elsewhere an earlier
+      // launch that this one may overlap (so not through the read-only path).  The factors
+      // are constant.
+      if (EXT && pp.scale == kScaleElements) y = fe_mul<F>(load_data<COHERENT>(f, false), x);
       else y = fe_reduce<F>(fe_mul_fixed<F>(x, ld_fe32(f), ld_fe32(f + 2)));
     } else if (last) {
       y = fe_canonical<F>(x);
