@@ -160,7 +160,8 @@ int zntt_ntt_device_columns(const zntt_twiddles* tw, const uint64_t* const* d_sr
  * is an 8 MiB array inside the library, held by every device that loads the
  * library until the process exits.  The first call on a device looks up that
  * array's device address (make it before any stream capture).  All calls
- * share the array: calls that overlap on the GPU race.  Larger transforms are
+ * of 2^12 elements and more share the array: those that overlap on the GPU race
+ * (smaller ones are one in-place pass and do not use it).  Larger transforms are
  * rejected with ZNTT_ERR_INVALID_ARGUMENT. */
 int zntt_ntt_device_inplace_noalloc(const zntt_twiddles* tw, uint64_t* d_data, int mode, void* stream);
 

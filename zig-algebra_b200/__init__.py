@@ -456,7 +456,7 @@ def ntt_device_inplace_noalloc(tw: DeviceTwiddles, d_data: int, mode: int = FORW
     For callers that must not allocate device memory while they transform
     (a fixed up-front memory budget, memory owned by another allocator, or a
     latency-critical path).  Its scratch is an 8 MiB array inside the library;
-    calls that overlap on the GPU share it and race."""
+    calls of 2^12 elements and more that overlap on the GPU share it and race."""
     _check(lib().zntt_ntt_device_inplace_noalloc(tw.handle, d_data, mode, stream or None))
 
 

@@ -21,8 +21,10 @@
 // cudaGetSymbolAddress (with that device current) and caches it; make that
 // first call before any stream capture.  All calls share the one array and it
 // keeps whatever the last call left in it; the transform overwrites every
-// element it reads, so nothing needs clearing, but calls that overlap on the
-// GPU (concurrent streams, or several host threads) race on the scratch.
+// element it reads, so nothing needs clearing, but calls of 2^12 elements and
+// more that overlap on the GPU (concurrent streams, or several host threads)
+// race on the scratch.  Up to 2^11 a transform is one in-place pass and does not
+// use it.
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -85,9 +87,13 @@ extern "C" int zntt_ntt_device_inplace_noalloc(const zntt_twiddles* tw, uint64_t
     scratch = static_cast<uint4*>(g_noalloc_scratch_addr[dev]);
   }
 
-  // The library's planner (a plan is a value; planning allocates nothing): one pass or two.
-  const Plan plan = log_n <= kRadix2MaxLog ? radix2_plan(log_n)
-                                           : make_plan(log_n, kDefaultShape, kShapes[kDefaultShape].log_tile - 1);
+  // The library's planner (a plan is a value; planning allocates nothing): one pass up to
+  // 2^11, which stays in place and leaves the scratch alone, so that calls of these sizes
+  // may overlap; beyond, two.  (Two radix-2 passes through the scratch would be faster at
+  // 2^9..2^11: BN254-Fr forward 10, 12 and 12 us against 12, 18 and 35, B200.)
+  const Plan plan = log_n <= (uint32_t)kShapes[kDefaultShape].log_tile || log_n > kRadix2MaxLog
+                        ? one_pass_plan(log_n)
+                        : radix2_plan(log_n);
   const uint32_t np = plan.np;
   const PassDesc* passes = plan.p;
 

@@ -247,6 +247,11 @@ Plan radix2_plan(uint32_t log_n) {
   return make_plan(log_n, k <= 7 ? kRadix2Shape : kRadix2Shape + 1, k);
 }
 
+Plan one_pass_plan(uint32_t log_n) {
+  return log_n <= 8 ? radix2_plan(log_n)
+                    : make_plan(log_n, kDefaultShape, kShapes[kDefaultShape].log_tile - 1);
+}
+
 Plan tuned_plan(int field, uint32_t log_n) {
   if (log_n >= 1 && log_n <= kRadix2MaxLog) return radix2_plan(log_n);
   return table_plan(field, log_n);

@@ -55,6 +55,9 @@ struct Plan {
 Plan make_plan(uint32_t log_n, int shape, uint32_t kmax);
 // The plan on the radix-2 shapes for 1 <= log_n <= kRadix2MaxLog.
 Plan radix2_plan(uint32_t log_n);
+// One pass for 1 <= log_n <= 11 (the default shape's tile), whatever the tuning table
+// holds: an in-place transform then needs no scratch.  Several passes beyond.
+Plan one_pass_plan(uint32_t log_n);
 // The radix-2 plan for the sizes it serves, else the plan the tuning table holds
 // for (field, log_n), else the default shape with kmax = log_tile - 1.
 Plan tuned_plan(int field, uint32_t log_n);
