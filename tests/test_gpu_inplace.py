@@ -65,3 +65,34 @@ def test_allocation_free_calls_may_overlap(z, log_n):
             torch.cuda.synchronize()
             for i, (x, w) in enumerate(zip(xs, wants)):
                 assert torch.equal(x, w), (F.name, i)
+
+
+@pytest.mark.parametrize("log_n", [8, 9, 10, 11])
+def test_no_wait_under_the_shipped_tuning_table(z, log_n):
+    """Whatever plan the tuning table holds, an in-place call without scratch neither waits nor
+    allocates up to 2^11, so a caller's graph can hold it."""
+    import os
+
+    import torch
+    z.tune_load(os.path.join(os.path.dirname(z.__file__), "tune", "b200.json"))
+    stream = torch.cuda.Stream()
+    try:
+        for F, fid in _fields(z):
+            _, root = O.primitive_root(fid, log_n)
+            _, stages = O.precompute_twiddles(fid, log_n, root)
+            with z.DeviceTwiddles(F, log_n, z.primitiveRootOfUnity(F, log_n)) as tw, torch.cuda.stream(stream):
+                for mode, inverse in ((z.FORWARD, False), (z.INVERSE, True)):
+                    x = _vec(z, F, 80 + log_n, 1 << log_n)
+                    torch.cuda.synchronize()
+                    want = _host(x)
+                    O.ntt_with_twiddles(fid, want, log_n, stages, inverse=inverse)
+                    before = z.pool_stats()["acquires"]
+                    graph = torch.cuda.CUDAGraph()
+                    with torch.cuda.graph(graph, stream=stream):
+                        z.ntt_device(tw, x.data_ptr(), x.data_ptr(), mode, stream=stream.cuda_stream)
+                    graph.replay()
+                    stream.synchronize()
+                    assert z.pool_stats()["acquires"] == before
+                    np.testing.assert_array_equal(_host(x), want, err_msg=f"{F.name} 2^{log_n} mode {mode}")
+    finally:
+        z.tune_clear()

@@ -254,10 +254,6 @@ Plan one_pass_plan(uint32_t log_n) {
 
 Plan tuned_plan(int field, uint32_t log_n) {
   if (log_n >= 1 && log_n <= kRadix2MaxLog) return radix2_plan(log_n);
-  return table_plan(field, log_n);
-}
-
-Plan table_plan(int field, uint32_t log_n) {
   const TuneEntry* best = nullptr;
   for (const TuneEntry& t : ctx().tune)
     if (t.field == field && t.log_n == log_n && (!best || t.us < best->us)) best = &t;
@@ -957,9 +953,9 @@ int zntt_ntt_device(const zntt_twiddles* tw, const uint64_t* d_src, uint64_t* d_
   const bool inverse = mode == ZNTT_INVERSE;
   const bool need_scratch = d_src == d_dst && tuned_plan(e->field, e->log_n).np > 1;
   if (need_scratch && !d_scratch) {
-    // One pass of the table's plan needs no scratch, so the call stays
-    // asynchronous (and can be captured) up to that plan's tile.
-    const Plan one = table_plan(e->field, e->log_n);
+    // One pass needs no scratch, so the call stays asynchronous (and can be
+    // captured) up to 2^11, whatever plan the tuning table holds.
+    const Plan one = one_pass_plan(e->log_n);
     if (one.np == 1)
       return run_plan(e->field, e, one, e->log_n, (const uint4*)d_src, (uint4*)d_dst, nullptr, inverse, inverse, st);
     // Borrow a pool buffer; it returns to the pool only after the stream has

@@ -61,8 +61,6 @@ Plan one_pass_plan(uint32_t log_n);
 // The radix-2 plan for the sizes it serves, else the plan the tuning table holds
 // for (field, log_n), else the default shape with kmax = log_tile - 1.
 Plan tuned_plan(int field, uint32_t log_n);
-// The same without the radix-2 shapes: one pass up to the shape's tile.
-Plan table_plan(int field, uint32_t log_n);
 // The tuned stage count for a given shape.
 uint32_t tuned_kmax(int field, uint32_t log_n, int shape);
 
