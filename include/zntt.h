@@ -419,9 +419,11 @@ uint64_t zntt_now_ns(void);
 
 /* ---- autotuner ------------------------------------------------------------------
  * Times every pass shape and stage count per pass for each log n in
- * [log_n_min, log_n_max] on this GPU, a forward and an inverse transform
- * each (one plan serves both directions), and keeps the fastest; plans use the
- * table from then on.  The table persists as JSON lines keyed by GPU name;
+ * [log_n_min, log_n_max] on this GPU, up to 2^16 the one-butterfly-per-thread
+ * passes beside them, a forward and an inverse transform each (one plan serves
+ * both directions), and keeps the fastest; plans use the table from then on.
+ * (A table saved by a version without those passes still decides the sizes it
+ * holds: tune again to have them considered.)  The table persists as JSON lines keyed by GPU name;
  * zntt_init loads the file named by ZNTT_TUNE_FILE when it exists. */
 int zntt_autotune(int field, uint32_t log_n_min, uint32_t log_n_max);
 int zntt_tune_save(const char* path);

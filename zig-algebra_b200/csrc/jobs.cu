@@ -527,6 +527,27 @@ int zntt_autotune(int field, uint32_t log_n_min, uint32_t log_n_max) {
     if (!rc) rc = pool_get((size_t)32 << L, &y);
     uint8_t seed[32] = {7};
     if (!rc) rc = zntt_random_elements(field, seed, (uint64_t*)x, (size_t)1 << L, nullptr);
+    // Microseconds per transform of a plan.  Each repetition is a forward and an
+    // inverse transform (the inverse's last pass also scales by 1/n): one plan serves
+    // both directions.
+    auto time_plan = [&](const Plan& plan) {
+      auto both = [&]() {
+        int r2 = run_plan(field, tw, plan, L, (const uint4*)x, (uint4*)y, nullptr, false, false, st);
+        if (!r2) r2 = run_plan(field, tw, plan, L, (const uint4*)x, (uint4*)y, nullptr, true, true, st);
+        return r2;
+      };
+      for (int w = 0; w < 2 && !rc; w++) rc = both();
+      const int reps = L >= 22 ? 5 : L >= 18 ? 20 : 50;
+      cudaEventRecord(e0, st);
+      for (int r = 0; r < reps && !rc; r++) rc = both();
+      cudaEventRecord(e1, st);
+      cudaError_t ce = cudaEventSynchronize(e1);
+      if (ce != cudaSuccess) rc = cuda_fail(ce, "autotune");
+      float ms = 0;
+      cudaEventElapsedTime(&ms, e0, e1);
+      return 1e3 * ms / (2 * reps);  // both directions averaged
+    };
+    const double radix2_us = !rc && L <= kRadix2MaxLog ? time_plan(radix2_plan(L)) : 0;
     for (int sh = 0; sh < kNumShapes && !rc; sh++) {
       const uint32_t lt = kShapes[sh].log_tile;
       TuneEntry best;
@@ -537,29 +558,14 @@ int zntt_autotune(int field, uint32_t log_n_min, uint32_t log_n_max) {
         if (plan.np == last_np && plan.p[0].k == last_k0) continue;  // same plan as a larger kmax
         last_np = plan.np;
         last_k0 = plan.p[0].k;
-        // Each repetition is a forward and an inverse transform (the inverse's
-        // last pass also scales by 1/n): one plan serves both directions.
-        auto both = [&]() {
-          int r2 = run_plan(field, tw, plan, L, (const uint4*)x, (uint4*)y, nullptr, false, false, st);
-          if (!r2) r2 = run_plan(field, tw, plan, L, (const uint4*)x, (uint4*)y, nullptr, true, true, st);
-          return r2;
-        };
-        for (int w = 0; w < 2 && !rc; w++) rc = both();
-        const int reps = L >= 22 ? 5 : L >= 18 ? 20 : 50;
-        cudaEventRecord(e0, st);
-        for (int r = 0; r < reps && !rc; r++) rc = both();
-        cudaEventRecord(e1, st);
-        cudaError_t ce = cudaEventSynchronize(e1);
-        if (ce != cudaSuccess) rc = cuda_fail(ce, "autotune");
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
-        const double us = 1e3 * ms / (2 * reps);  // per transform, both directions averaged
+        const double us = time_plan(plan);
         if (!rc && us < best.us) {
           best.field = field;
           best.log_n = L;
           best.shape = sh;
           best.kmax = kmax;
           best.us = us;
+          best.radix2_us = radix2_us;
         }
       }
       if (!rc) {
@@ -579,7 +585,8 @@ int zntt_autotune(int field, uint32_t log_n_min, uint32_t log_n_max) {
   return rc;
 }
 
-// One entry per line: {"gpu": "...", "field": F, "log_n": L, "shape": S, "kmax": K, "us": T}
+// One entry per line: {"gpu": "...", "field": F, "log_n": L, "shape": S, "kmax": K, "us": T}, and
+// "radix2_us": T2 where the radix-2 plan was timed too.
 int zntt_tune_save(const char* path) {
   clear_error();
   if (!path) return set_error(ZNTT_ERR_INVALID_ARGUMENT, "null path");
@@ -609,8 +616,10 @@ int zntt_tune_save(const char* path) {
     firstl = false;
   }
   for (const TuneEntry& t : c.tune) {
-    std::fprintf(f, "%s {\"gpu\": \"%s\", \"field\": %d, \"log_n\": %u, \"shape\": %d, \"kmax\": %u, \"us\": %.3f}",
+    std::fprintf(f, "%s {\"gpu\": \"%s\", \"field\": %d, \"log_n\": %u, \"shape\": %d, \"kmax\": %u, \"us\": %.3f",
                  firstl ? "" : ",\n", c.gpu_name.c_str(), t.field, t.log_n, t.shape, t.kmax, t.us);
+    if (t.radix2_us > 0) std::fprintf(f, ", \"radix2_us\": %.3f", t.radix2_us);
+    std::fprintf(f, "}");
     firstl = false;
   }
   std::fprintf(f, "\n]\n");
@@ -638,6 +647,8 @@ int zntt_tune_load(const char* path) {
     if (!q || std::sscanf(q, "\"field\": %d, \"log_n\": %u, \"shape\": %d, \"kmax\": %u, \"us\": %lf", &t.field,
                           &t.log_n, &t.shape, &t.kmax, &t.us) != 5)
       continue;
+    const char* r2 = std::strstr(q, "\"radix2_us\":");
+    if (r2 && std::sscanf(r2, "\"radix2_us\": %lf", &t.radix2_us) != 1) continue;
     if (t.shape < 0 || t.shape >= kNumShapes || t.kmax < 2 || t.kmax > (uint32_t)kShapes[t.shape].log_tile) continue;
     c.tune.erase(std::remove_if(c.tune.begin(), c.tune.end(),
                                 [&](const TuneEntry& u) {

@@ -64,10 +64,11 @@ constexpr int kNumShapes = 5;
 constexpr PassShape kShapes[kNumShapes + 2] = {{11, 256, 3}, {10, 256, 3}, {9, 128, 6}, {8, 64, 12},
                                                {9, 128, 7},  {7, 64, 8},   {8, 128, 4}};
 constexpr int kRadix2Shape = kNumShapes;
-// Plain transforms up to this size run on the radix-2 shapes.  Both ways, two
-// transforms (forward and inverse) of BN254-Fr in us, B200: 2^10 24.6 against 37.1
-// with the tuned radix-4 passes, 2^14 31.7 / 47.1, 2^16 43.0 / 51.2, and from 2^17
-// on the radix-4 passes are as fast or faster (63.5 / 63.6, 2^18 106 / 102).
+// Plain transforms up to this size run on the radix-2 shapes, unless the tuning table
+// holds a faster plan.  Both ways, two transforms (forward and inverse) of BN254-Fr in
+// us, B200: 2^10 24.6 against 38.9 with the tuned radix-4 passes, 2^14 30.9 / 47.2,
+// 2^16 42.7 / 51.3 (BLS12-381-Fr 22.6 / 35.9, 28.7 / 45.1, 41.0 / 51.2), and from 2^17
+// on the radix-4 passes are as fast or faster (BN254-Fr 63.5 / 63.6, 2^18 106 / 102).
 constexpr uint32_t kRadix2MaxLog = 16;
 // The shape of persistent launches (batches and the server's slices): the
 // 7-CTA 2^9 tile runs the mixed 520-transform batch in 2.22 ms, the 2^11 tile in

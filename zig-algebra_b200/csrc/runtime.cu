@@ -253,11 +253,13 @@ Plan one_pass_plan(uint32_t log_n) {
 }
 
 Plan tuned_plan(int field, uint32_t log_n) {
-  if (log_n >= 1 && log_n <= kRadix2MaxLog) return radix2_plan(log_n);
   const TuneEntry* best = nullptr;
   for (const TuneEntry& t : ctx().tune)
     if (t.field == field && t.log_n == log_n && (!best || t.us < best->us)) best = &t;
-  if (best) return make_plan(log_n, best->shape, best->kmax);
+  const bool radix2 = log_n >= 1 && log_n <= kRadix2MaxLog;
+  if (best && !(radix2 && best->radix2_us > 0 && best->radix2_us <= best->us))
+    return make_plan(log_n, best->shape, best->kmax);
+  if (radix2) return radix2_plan(log_n);
   return make_plan(log_n, kDefaultShape, kShapes[kDefaultShape].log_tile - 1);
 }
 

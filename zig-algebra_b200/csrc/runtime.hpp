@@ -58,8 +58,9 @@ Plan radix2_plan(uint32_t log_n);
 // One pass for 1 <= log_n <= 11 (the default shape's tile), whatever the tuning table
 // holds: an in-place transform then needs no scratch.  Several passes beyond.
 Plan one_pass_plan(uint32_t log_n);
-// The radix-2 plan for the sizes it serves, else the plan the tuning table holds
-// for (field, log_n), else the default shape with kmax = log_tile - 1.
+// The fastest plan the tuning table holds for (field, log_n), the radix-2 plan among
+// them where the tuner timed it; without entries the radix-2 plan for the sizes it
+// serves, else the default shape with kmax = log_tile - 1.
 Plan tuned_plan(int field, uint32_t log_n);
 // The tuned stage count for a given shape.
 uint32_t tuned_kmax(int field, uint32_t log_n, int shape);
@@ -71,6 +72,7 @@ struct TuneEntry {
   int shape = 0;
   uint32_t kmax = 0;
   double us = 0;
+  double radix2_us = 0;  // the radix-2 plan's time in the same tuning run (0: not timed)
 };
 
 // Caching device allocator: freed buffers are kept by exact size for reuse.
