@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -186,12 +187,15 @@ int root_wait_begin(uint64_t subtrees, RootWait* out) {
 
 int root_wait(const RootWait& w, cudaStream_t st, uint8_t* root_out, const char* what) {
   // The root arrives while the kernel's launch is still being retired: reading it
-  // as it lands saves a copy and most of a stream synchronisation per round.  A
-  // launch that failed never writes it, which the stream's status tells.
-  for (uint32_t spin = 1; *w.seq != w.value; spin++) {
-    if (spin % 4096) continue;
-    const cudaError_t e = cudaStreamQuery(st);
-    if (e == cudaErrorNotReady) continue;
+  // as it lands saves a copy and most of a stream synchronisation per round, which
+  // counts in the rounds of some 30 us.  A longer wait goes on in a synchronisation,
+  // which sleeps or yields where the process asked for that (cudaSetDeviceFlags)
+  // and tells a launch that failed.
+  using clock = std::chrono::steady_clock;
+  const clock::time_point until = clock::now() + std::chrono::microseconds(200);
+  while (*w.seq != w.value) {
+    if (clock::now() < until) continue;
+    const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, what);
     if (*w.seq != w.value) return set_error(ZNTT_ERR_DEVICE, std::string(what) + ": no root");
   }
