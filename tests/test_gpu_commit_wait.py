@@ -4,6 +4,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import time
 
 import pytest
 
@@ -46,3 +47,27 @@ def test_a_long_wait_leaves_the_core(z):
     wall, cpu = map(float, out.stdout.split())
     assert wall > 30 * 1e-3  # milliseconds each, so that the bound says something
     assert cpu < 0.5 * wall, (wall, cpu)
+
+
+def test_a_larger_commitment_does_not_wait_for_other_streams(z):
+    """A commitment larger than any before it neither frees nor allocates: it returns while
+    another stream is still busy."""
+    import torch
+    z.shutdown()
+    z.init(0)
+    F, L = z.GOLDILOCKS, 26
+    layer = torch.zeros(1 << L, dtype=torch.int64, device="cuda")
+    nodes = torch.empty(32 << L, dtype=torch.uint8, device="cuda")
+    mine, other = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    z.fri_commit_layer(F, layer.data_ptr(), 22, nodes.data_ptr(), stream=mine.cuda_stream)  # the same kernels
+    with torch.cuda.stream(other):
+        torch.cuda._sleep(2_000_000_000)  # about a second
+        busy = torch.cuda.Event()
+        busy.record()
+    t0 = time.perf_counter()
+    root = z.fri_commit_layer(F, layer.data_ptr(), L, nodes.data_ptr(), stream=mine.cuda_stream)
+    took = time.perf_counter() - t0
+    assert not busy.query() and took < 0.5, took
+    torch.cuda.synchronize()
+    assert root == z.fri_commit_layer(F, layer.data_ptr(), L, nodes.data_ptr(), stream=mine.cuda_stream)

@@ -266,6 +266,9 @@ cudaError_t build_tree(const Src& src, uint4* nodes, uint64_t h, cudaStream_t st
 // and 41 us, 2^20 72 and 67, 2^24 560 and 516; below it one launch is the faster
 // (2^16 33.9 us, 43.5 in launches; lines at 2^19 and 2^21 are no faster; B200).
 constexpr uint64_t kOwnLaunchWidth = (uint64_t)1 << 17;
+// So a tree_kernel's level has at most half of that, 128 subtrees in groups of sixteen: 8
+// counters for the first level of groups and one for the last.
+static_assert(kOwnLaunchWidth / 2 / (2 * kThreads) <= 256 && 256 / 16 + 1 <= kTreeTickets, "a counter for every group");
 
 // tree_kernel over the level of width w, made by the launch before it on `st`.
 cudaError_t launch_node_tree(uint4* nodes, uint64_t w, uint32_t* tickets, const RootOut& out, cudaStream_t st) {
@@ -324,7 +327,7 @@ int commit_tree(const Src& src, uint4* nodes, uint64_t h, uint8_t* root_out, cud
     return ce == cudaSuccess ? ZNTT_OK : cuda_fail(ce, what);
   }
   RootWait wait;
-  int rc = root_wait_begin(h / (2 * kThreads), &wait);
+  int rc = root_wait_begin(&wait);
   if (rc) return rc;
   const cudaError_t ce =
       build_tree_root(src, nodes, h, wait.tickets, RootOut{static_cast<uint4*>(wait.root), wait.seq, wait.value}, st);

@@ -157,21 +157,18 @@ struct PoolBuf {
 // commitment roots
 // ---------------------------------------------------------------------------
 
-int root_wait_begin(uint64_t subtrees, RootWait* out) {
+int root_wait_begin(RootWait* out) {
   Context& c = ctx();
-  // subtrees / 16 counters for the first level of sixteens, then a sixteenth of
-  // those, ..., and one for each level of fewer than sixteen.
-  const size_t words = subtrees / 15 + 16;
-  if (words > c.tickets_words) {
-    if (c.tickets) cudaFree(c.tickets);
-    c.tickets = nullptr;
-    c.tickets_words = 0;
-    const size_t get = std::max<size_t>(words, 4096);
-    ZCHECK(cudaMalloc((void**)&c.tickets, get * 4), "tree counters");
-    cudaError_t e = cudaMemsetAsync(c.tickets, 0, get * 4, c.stream);
+  if (!c.tickets) {
+    uint32_t* t = nullptr;
+    ZCHECK(cudaMalloc((void**)&t, kTreeTickets * 4), "tree counters");
+    cudaError_t e = cudaMemsetAsync(t, 0, kTreeTickets * 4, c.stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
-    if (e != cudaSuccess) return cuda_fail(e, "tree counters");
-    c.tickets_words = get;
+    if (e != cudaSuccess) {
+      cudaFree(t);
+      return cuda_fail(e, "tree counters");
+    }
+    c.tickets = t;
   }
   if (!c.root_host) {
     ZCHECK(cudaHostAlloc(&c.root_host, 64, cudaHostAllocDefault), "pinned root");
@@ -684,7 +681,6 @@ int zntt_shutdown(void) {
   c.regs.clear();
   if (c.tickets) cudaFree(c.tickets);
   c.tickets = nullptr;
-  c.tickets_words = 0;
   if (c.root_host) cudaFreeHost(c.root_host);
   c.root_host = nullptr;
   c.pool.release_all();

@@ -117,7 +117,6 @@ struct Context {
   std::string gpu_name;
   cudaStream_t pipe[3] = {nullptr, nullptr, nullptr};  // streams of the pipelined host API
   uint32_t* tickets = nullptr;  // zeroed counters of the commitments' trees (between calls all zero)
-  size_t tickets_words = 0;
   void* root_host = nullptr;    // pinned: a commitment's root (32 bytes), then its sequence number
   uint32_t root_seq = 0;
   std::vector<TuneEntry> tune;  // best kmax per (field, log_n, shape) on this GPU
@@ -143,15 +142,16 @@ int run_plan(int field, const TwEntry* tw, const Plan& plan, uint32_t log_n, con
              uint4* d_scratch, bool inverse, bool scale, cudaStream_t st);
 
 // A commitment that the caller waits for (the library lock held from begin to
-// wait, so one at a time): counters for `subtrees` subtrees, and pinned memory
-// that the kernel writes the root and then `value` (at seq) to.
+// wait, so one at a time): counters for the groups of subtrees of one launch, and
+// pinned memory that the kernel writes the root and then `value` (at seq) to.
+constexpr uint32_t kTreeTickets = 64;
 struct RootWait {
   uint32_t* tickets = nullptr;
   void* root = nullptr;
   volatile uint32_t* seq = nullptr;
   uint32_t value = 0;
 };
-int root_wait_begin(uint64_t subtrees, RootWait* out);
+int root_wait_begin(RootWait* out);
 int root_wait(const RootWait& w, cudaStream_t st, uint8_t* root_out, const char* what);
 
 // Pool buffer helpers shared by the translation units.
