@@ -83,12 +83,14 @@ __device__ __forceinline__ void small_butterfly(uint64_t& u, uint64_t& v, bool m
 // One tile of one pass, for what small_tile.cuh does not take: transforms below
 // 2^12 and caller tables whose entries of index 0 are not one.  PAD: the first
 // pass reads natural indices at or beyond pp.src_len as zeros (a zero-padded
-// input that is not stored).
-template <class SF, bool PAD>
+// input that is not stored).  FULL: the tile is the whole 2^12, so no bound checks
+// (in place without scratch at 2^12, inverse: Goldilocks 24.7 us with them and 22.6
+// without, BabyBear 16.5 and 14.4; B200).
+template <class SF, bool PAD, bool FULL>
 __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t blk, uint64_t* sm) {
   constexpr uint32_t TILE_MAX = 1u << kSmallLogTile, THREADS = kSmallThreads;
   const uint32_t k = pp.k, c = pp.c, C = 1u << c;
-  const uint32_t tile = 1u << (k + c);
+  const uint32_t tile = FULL ? TILE_MAX : 1u << (k + c);
   const uint32_t tid = threadIdx.x;
   uint32_t hi_base = 0, m0 = 0, col0 = 0;
   if (pp.first) {
@@ -103,7 +105,7 @@ __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t bl
 #pragma unroll
   for (uint32_t q = 0; q < TILE_MAX / THREADS; q++) {
     const uint32_t e = tid + q * THREADS;
-    if (e < tile) {
+    if (FULL || e < tile) {
       const uint32_t col = e & (C - 1), row = e >> c;
       uint32_t g, t;
       if (pp.first) {
@@ -125,7 +127,7 @@ __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t bl
 #pragma unroll
     for (uint32_t q = 0; q < TILE_MAX / 2 / THREADS; q++) {
       const uint32_t b = tid + q * THREADS;
-      if (b < tile / 2) {
+      if (FULL || b < tile / 2) {
         const uint32_t col = b & (C - 1), t0 = (b >> c) << 1;
         const uint32_t jg = pp.first ? 0 : m0 + col;
         const uint32_t e0 = (t0 << c) | col, e1 = e0 + C;
@@ -147,7 +149,7 @@ __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t bl
 #pragma unroll
     for (uint32_t q = 0; q < TILE_MAX / 4 / THREADS; q++) {
       const uint32_t ga = tid + q * THREADS;
-      if (ga < tile / 4) {
+      if (FULL || ga < tile / 4) {
         const uint32_t col = ga & (C - 1), g = ga >> c;
         const uint32_t j = g & (h - 1);
         const uint32_t t0 = ((g >> (i - 1)) << (i + 1)) | j;
@@ -181,7 +183,7 @@ __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t bl
 #pragma unroll
   for (uint32_t q = 0; q < TILE_MAX / THREADS; q++) {
     const uint32_t e = tid + q * THREADS;
-    if (e < tile) {
+    if (FULL || e < tile) {
       const uint32_t col = e & (C - 1), row = e >> c;
       const uint32_t g = pp.first ? (rev_bits_small(col0 + col, xcols_log) << k) + row
                                   : hi_base + (row << pp.S) + m0 + col;
@@ -192,10 +194,10 @@ __device__ __forceinline__ void small_pass_body(const SmallPass& pp, uint32_t bl
   }
 }
 
-template <class SF>
+template <class SF, bool FULL>
 __global__ void __launch_bounds__(kSmallThreads) small_pass_kernel(SmallPass pp) {
   __shared__ uint64_t sm[1u << kSmallLogTile];
-  small_pass_body<SF, false>(pp, blockIdx.x, sm);
+  small_pass_body<SF, false, FULL>(pp, blockIdx.x, sm);
 }
 
 // The same pass over many columns of one size: column blockIdx.y reads
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(kSmallThreads) small_pass_cols_kernel(SmallPas
   SmallPass q = pp;
   q.src = srcs[blockIdx.y];
   q.dst = dsts[blockIdx.y];
-  small_pass_body<SF, true>(q, blockIdx.x, sm);
+  small_pass_body<SF, true, false>(q, blockIdx.x, sm);
 }
 
 // Four CTAs per SM (64 registers, no spill): 2^24 Goldilocks forward 0.398 ms with
@@ -362,9 +364,15 @@ __global__ void small_bit_reverse_kernel(const uint64_t* __restrict__ src, uint6
 
 int grid_for(uint64_t count) { return (int)std::min<uint64_t>((count + 255) / 256, 148 * 16); }
 
+template <class SF>
+static void launch_small_pass_t(const SmallPass& pp, unsigned tiles, cudaStream_t st) {
+  if (pp.k + pp.c == (uint32_t)kSmallLogTile) small_pass_kernel<SF, true><<<tiles, kSmallThreads, 0, st>>>(pp);
+  else small_pass_kernel<SF, false><<<tiles, kSmallThreads, 0, st>>>(pp);
+}
+
 cudaError_t launch_small_pass(int field, const SmallPass& pp, uint64_t tiles, cudaStream_t st) {
-  if (field == kGoldilocksField) small_pass_kernel<Goldilocks><<<(unsigned)tiles, kSmallThreads, 0, st>>>(pp);
-  else small_pass_kernel<BabyBear><<<(unsigned)tiles, kSmallThreads, 0, st>>>(pp);
+  if (field == kGoldilocksField) launch_small_pass_t<Goldilocks>(pp, (unsigned)tiles, st);
+  else launch_small_pass_t<BabyBear>(pp, (unsigned)tiles, st);
   return cudaGetLastError();
 }
 
