@@ -1,0 +1,62 @@
+"""What the library does when device memory runs out, and what it keeps idle.  Needs a B200."""
+from __future__ import annotations
+
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+GIB = 1 << 30
+
+
+@pytest.fixture(scope="module")
+def z(zntt):
+    zntt.init(0)
+    return zntt
+
+
+@pytest.fixture
+def fresh(z):
+    """The library with nothing cached, before and after."""
+    import torch
+    z.shutdown()
+    z.init(0)
+    torch.cuda.empty_cache()
+    yield z
+    z.shutdown()
+    z.init(0)
+    torch.cuda.empty_cache()
+
+
+def _fill(leave):
+    """A torch buffer that takes all free device memory but `leave` bytes."""
+    import torch
+    torch.cuda.synchronize()
+    free, _ = torch.cuda.mem_get_info()
+    return torch.empty(free - leave, dtype=torch.uint8, device="cuda")
+
+
+def _roundtrip(z, F, log_n):
+    import torch
+    x = torch.zeros(4 << log_n, dtype=torch.int64, device="cuda")
+    y, w = torch.zeros_like(x), torch.zeros_like(x)
+    torch.cuda.synchronize()
+    with z.DeviceTwiddles(F, log_n, z.primitiveRootOfUnity(F, log_n)) as tw:
+        z.random_elements(F, 9, x.data_ptr(), 1 << log_n)
+        z.ntt_device(tw, x.data_ptr(), y.data_ptr(), z.FORWARD)
+        z.ntt_device(tw, y.data_ptr(), w.data_ptr(), z.INVERSE)
+        torch.cuda.synchronize()
+    assert torch.equal(x, w) and not torch.equal(x, y)
+
+
+def test_a_refused_allocation_is_not_the_next_calls_error(fresh):
+    z, F = fresh, fresh.BN254_FR
+    _roundtrip(z, F, 10)  # the slabs of small buffers are there before memory is taken
+    filler = _fill(2 * GIB)
+    try:
+        with pytest.raises(z.OutOfMemory):
+            z.DeviceTwiddles(F, 27, z.primitiveRootOfUnity(F, 27))
+        _roundtrip(z, F, 10)
+    finally:
+        del filler

@@ -34,6 +34,9 @@ int set_error(int status, const std::string& msg) {
 void clear_error() { g_last_error.clear(); }
 
 int cuda_fail(cudaError_t e, const char* what) {
+  // The runtime also keeps e as this thread's last error: left there, a refused
+  // allocation would be taken for the next call's failed launch.
+  cudaGetLastError();
   std::string m = std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
   if (e == cudaErrorMemoryAllocation) return set_error(ZNTT_ERR_OUT_OF_MEMORY, m);
   return set_error(ZNTT_ERR_DEVICE, m);
