@@ -60,3 +60,24 @@ def test_a_refused_allocation_is_not_the_next_calls_error(fresh):
         _roundtrip(z, F, 10)
     finally:
         del filler
+
+
+def test_caller_tables_leave_two_vectors_in_the_pool(fresh):
+    """A host call with the caller's own table keeps what any host call does: its two vectors."""
+    z, F, log_n = fresh, fresh.BN254_FR, 18
+    tab = z.precomputeTwiddles(F, log_n, z.primitiveRootOfUnity(F, log_n))
+    own = [np.array(s, copy=True) for s in tab]
+    z.freeTwiddles(F, tab)
+    z.shutdown()
+    z.init(0)
+    before = z.pool_stats()
+    data = np.zeros((1 << log_n, 4), dtype=np.uint64)
+    data[:, 0] = np.arange(1 << log_n)
+    keep = data.copy()
+    for _ in range(3):
+        z.nttWithTwiddles(F, data, log_n, own)
+        z.inttWithTwiddles(F, data, log_n, own)
+    assert np.array_equal(data, keep)
+    after = z.pool_stats()
+    assert after["cached_bytes"] - before["cached_bytes"] == 2 * (32 << log_n)
+    assert after["device_mallocs"] - before["device_mallocs"] == 2

@@ -336,7 +336,6 @@ static size_t table_bytes(uint32_t log_n) { return (size_t)64 << log_n; }
 static void free_entry(TwEntry* e) {
   Context& c = ctx();
   if (e->d_table) cudaFree(e->d_table);
-  if (e->upload) c.pool.release(e->upload, e->upload_bytes);
   c.all_tables.erase(std::remove(c.all_tables.begin(), c.all_tables.end(), e), c.all_tables.end());
   for (auto it = c.tw_by_key.begin(); it != c.tw_by_key.end(); ++it) {
     if (it->second == e) {
@@ -452,7 +451,10 @@ void release_table(TwEntry* e) {
 }
 
 // Builds a device table from a caller's host table that the library did not
-// make (or no longer recognises), with zig-ntt's exact per-stage semantics.
+// make (or no longer recognises), with zig-ntt's exact per-stage semantics.  The
+// entries as given pass through a pool buffer that is back in the pool on return,
+// for the same stream to use next: the caller holds the lock until that stream has
+// finished.
 static int upload_foreign_table(int field, uint32_t log_n, const zntt_stage* stages, TwEntry** out) {
   Context& c = ctx();
   const HostField& F = host_field(field);
@@ -466,8 +468,8 @@ static int upload_foreign_table(int field, uint32_t log_n, const zntt_stage* sta
     delete e;
     return cuda_fail(ce, "foreign twiddle table");
   }
-  e->upload_bytes = (size_t)32 << log_n;
-  int rc = pool_get(e->upload_bytes, &e->upload);
+  PoolBuf upload;
+  int rc = upload.get((size_t)32 << log_n);
   if (rc) {
     cudaFree(e->d_table);
     delete e;
@@ -477,16 +479,15 @@ static int upload_foreign_table(int field, uint32_t log_n, const zntt_stage* sta
   for (uint32_t s = 0; s < log_n; s++) {
     if (!F.is_one(stages[s].ptr)) e->tw0_one = false;
     if (ce == cudaSuccess)
-      ce = cudaMemcpyAsync((uint4*)e->upload + 2 * (((size_t)1 << s) - 1), stages[s].ptr, ((size_t)1 << s) * 32,
+      ce = cudaMemcpyAsync((uint4*)upload.p + 2 * (((size_t)1 << s) - 1), stages[s].ptr, ((size_t)1 << s) * 32,
                            cudaMemcpyHostToDevice, c.stream);
   }
   uint64_t ninv[4];
   n_inverse(field, log_n, ninv);
-  if (ce == cudaSuccess) ce = launch_twiddle_pairs(field, (const uint4*)e->upload, ninv, e->d_table, log_n, c.stream);
+  if (ce == cudaSuccess) ce = launch_twiddle_pairs(field, (const uint4*)upload.p, ninv, e->d_table, log_n, c.stream);
   if (ce != cudaSuccess) {
     cudaStreamSynchronize(c.stream);
     cudaFree(e->d_table);
-    pool_put(e->upload, e->upload_bytes);
     delete e;
     return cuda_fail(ce, "foreign twiddle upload");
   }

@@ -27,8 +27,6 @@ struct TwEntry {
   bool tw0_one = true;              // every stage's entry 0 equals one
   bool foreign = false;             // uploaded from a caller's table, not derived from a root
   uint64_t last_use = 0;
-  void* upload = nullptr;           // a foreign table's entries as given (pool buffer, released with the table)
-  size_t upload_bytes = 0;
   const uint4* n_inv() const { return d_table + 4 * (((size_t)1 << log_n) - 1); }
 };
 
