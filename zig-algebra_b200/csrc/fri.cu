@@ -86,7 +86,7 @@ int fold_table(int field, uint32_t log_n, const uint4** out) {
   FoldTable t;
   const uint64_t count = 1ull << (log_n - 1);
   t.bytes = count * 64;
-  cudaError_t ce = cudaMalloc((void**)&t.d, t.bytes);
+  cudaError_t ce = device_malloc((void**)&t.d, t.bytes);
   if (ce != cudaSuccess) return cuda_fail(ce, "fold table");
   rc = powers_device(field, ginv, half_inv, t.d, count, true, ctx().stream);
   if (rc) {

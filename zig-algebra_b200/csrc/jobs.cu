@@ -40,7 +40,7 @@ int acquire_coset_tab(int field, uint32_t log_in, const uint64_t* shift, CosetTa
   t->log_in = log_in;
   std::memcpy(t->shift, shift, 32);
   t->bytes = ((size_t)64) << log_in;
-  cudaError_t ce = cudaMalloc((void**)&t->d, t->bytes);
+  cudaError_t ce = device_malloc((void**)&t->d, t->bytes);
   if (ce != cudaSuccess) {
     delete t;
     return cuda_fail(ce, "coset scale table");
@@ -73,10 +73,20 @@ int acquire_coset_tab(int field, uint32_t log_in, const uint64_t* shift, CosetTa
 
 // Tables stay resident when their last user lets go (a cudaFree would
 // synchronise the device behind work in flight, and the next extension of the
-// same size would rebuild the table); zntt_shutdown frees them.
+// same size would rebuild the table); a full device (drop_idle_coset_tabs) or
+// zntt_shutdown frees them.
 void release_coset_tab(CosetTab* t) {
   if (!t) return;
   if (t->refs > 0) t->refs--;
+}
+
+void drop_idle_coset_tabs() {
+  auto idle = std::stable_partition(g_coset_tabs.begin(), g_coset_tabs.end(), [](CosetTab* t) { return t->refs > 0; });
+  for (auto it = idle; it != g_coset_tabs.end(); ++it) {
+    cudaFree((*it)->d);
+    delete *it;
+  }
+  g_coset_tabs.erase(idle, g_coset_tabs.end());
 }
 
 void free_coset_tabs() {
@@ -319,10 +329,10 @@ int zntt_batch_create(int field, const zntt_job* jobs, size_t n_jobs, int shape,
     }
   }
   b->ctl_words = 2 + b->passes.size();
-  cudaError_t ce = cudaMalloc((void**)&b->d_passes, std::max<size_t>(1, b->passes.size()) * sizeof(BatchPass));
+  cudaError_t ce = device_malloc((void**)&b->d_passes, std::max<size_t>(1, b->passes.size()) * sizeof(BatchPass));
   if (ce == cudaSuccess)
-    ce = cudaMalloc((void**)&b->d_items, std::max<size_t>(1, b->items.size()) * sizeof(BatchItem));
-  if (ce == cudaSuccess) ce = cudaMalloc((void**)&b->d_ctl, b->ctl_words * 4);
+    ce = device_malloc((void**)&b->d_items, std::max<size_t>(1, b->items.size()) * sizeof(BatchItem));
+  if (ce == cudaSuccess) ce = device_malloc((void**)&b->d_ctl, b->ctl_words * 4);
   if (ce == cudaSuccess && !b->passes.empty())
     ce = cudaMemcpyAsync(b->d_passes, b->passes.data(), b->passes.size() * sizeof(BatchPass), cudaMemcpyHostToDevice,
                          st);

@@ -19,6 +19,8 @@ struct CosetTab {
 };
 int acquire_coset_tab(int field, uint32_t log_in, const uint64_t* shift, CosetTab** out, cudaStream_t st);
 void release_coset_tab(CosetTab* t);
+// Frees the tables without a user.
+void drop_idle_coset_tabs();
 void free_coset_tabs();
 
 // The passes of one job, in order, with the buffers they run between.

@@ -71,13 +71,7 @@ cudaError_t BufferPool::acquire(size_t bytes, void** out) {
     if (slabs_.empty() || slab_used_ + need > slabs_.back().second) {
       void* slab = nullptr;
       mallocs_++;
-      cudaError_t e = cudaMalloc(&slab, kSlabBytes);
-      if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        trim();
-        mallocs_++;
-        e = cudaMalloc(&slab, kSlabBytes);
-      }
+      cudaError_t e = device_malloc(&slab, kSlabBytes);
       if (e != cudaSuccess) {
         cudaGetLastError();
         slab = nullptr;
@@ -93,14 +87,7 @@ cudaError_t BufferPool::acquire(size_t bytes, void** out) {
     }
   }
   mallocs_++;
-  cudaError_t e = cudaMalloc(out, bytes);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    trim();
-    mallocs_++;
-    e = cudaMalloc(out, bytes);
-  }
-  return e;
+  return device_malloc(out, bytes);
 }
 
 bool BufferPool::in_slab(const void* p) const {
@@ -363,6 +350,18 @@ static void evict_tables(size_t need) {
   }
 }
 
+cudaError_t device_malloc(void** out, size_t bytes) {
+  cudaError_t e = cudaMalloc(out, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  Context& c = ctx();
+  c.pool.trim();
+  evict_tables(c.table_cache_budget + 1);
+  small_drop_idle();
+  drop_idle_coset_tabs();
+  return cudaMalloc(out, bytes);
+}
+
 // pw[0][i] = base^i, pw[1][i] = base^(1024 i), pw[2][i] = base^(2^20 i), i < 1024:
 // the three tables the twiddle and powers kernels multiply together.
 void host_power_tables(int field, const uint64_t* base, std::vector<uint64_t>& pw) {
@@ -414,13 +413,7 @@ int acquire_table(int field, uint32_t log_n, const uint64_t* root, TwEntry** out
   std::memcpy(e->root, root, 32);
   e->bytes = table_bytes(log_n);
   evict_tables(e->bytes);
-  cudaError_t ce = cudaMalloc((void**)&e->d_table, e->bytes);
-  if (ce == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    c.pool.trim();
-    evict_tables(c.table_cache_budget + 1);  // drop every idle table
-    ce = cudaMalloc((void**)&e->d_table, e->bytes);
-  }
+  cudaError_t ce = device_malloc((void**)&e->d_table, e->bytes);
   if (ce != cudaSuccess) {
     delete e;
     return cuda_fail(ce, "twiddle table");
@@ -463,7 +456,7 @@ static int upload_foreign_table(int field, uint32_t log_n, const zntt_stage* sta
   e->log_n = log_n;
   e->foreign = true;
   e->bytes = table_bytes(log_n);
-  cudaError_t ce = cudaMalloc((void**)&e->d_table, e->bytes);
+  cudaError_t ce = device_malloc((void**)&e->d_table, e->bytes);
   if (ce != cudaSuccess) {
     delete e;
     return cuda_fail(ce, "foreign twiddle table");

@@ -111,7 +111,9 @@ struct Context {
   std::vector<Registration> regs;
   BufferPool pool;
   uint64_t clock = 0;
-  size_t table_cache_budget = (size_t)16 << 30;  // unreferenced root tables kept up to this
+  // Unreferenced root tables are kept up to this: two of 2^28 elements (a forward and an
+  // inverse root).  Freeing one and allocating the next takes 0.65 s at that size.
+  size_t table_cache_budget = (size_t)33 << 30;
   std::string gpu_name;
   cudaStream_t pipe[3] = {nullptr, nullptr, nullptr};  // streams of the pipelined host API
   uint32_t* tickets = nullptr;  // zeroed counters of the commitments' trees (between calls all zero)
@@ -152,6 +154,9 @@ struct RootWait {
 int root_wait_begin(RootWait* out);
 int root_wait(const RootWait& w, cudaStream_t st, uint8_t* root_out, const char* what);
 
+// cudaMalloc under the library lock.  On a full device the library's own idle memory
+// goes first (cached pool buffers, tables without a user), then it tries again.
+cudaError_t device_malloc(void** out, size_t bytes);
 // Pool buffer helpers shared by the translation units.
 int pool_get(size_t bytes, void** out);
 void pool_put(void* p, size_t bytes);

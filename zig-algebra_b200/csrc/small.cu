@@ -558,7 +558,7 @@ int small_acquire(int field, uint32_t log_n, uint64_t root, SmallTable** out) {
   e->n_inv = H.inv(((uint64_t)1 << log_n) % H.p);
   e->bytes = small_entries(log_n) * 8;
   small_evict(e->bytes);
-  cudaError_t ce = cudaMalloc((void**)&e->d_table, e->bytes);
+  cudaError_t ce = device_malloc((void**)&e->d_table, e->bytes);
   if (ce != cudaSuccess) {
     delete e;
     return cuda_fail(ce, "twiddle table");
@@ -608,7 +608,7 @@ int small_upload_foreign(int field, uint32_t log_n, const zntt_stage* stages, Sm
   e->foreign = true;
   e->n_inv = small_host(field).inv(((uint64_t)1 << log_n) % small_host(field).p);
   e->bytes = small_entries(log_n) * 8;
-  cudaError_t ce = cudaMalloc((void**)&e->d_table, e->bytes);
+  cudaError_t ce = device_malloc((void**)&e->d_table, e->bytes);
   if (ce != cudaSuccess) {
     delete e;
     return cuda_fail(ce, "foreign twiddle table");
@@ -1055,7 +1055,7 @@ int small_fold_params(int field, uint32_t log_table, const uint64_t* alpha, cons
     small_primitive_root(field, log_table, g);
     const uint64_t count = 1ull << (log_table - 1);
     uint64_t* tab = nullptr;
-    cudaError_t ce = cudaMalloc((void**)&tab, count * 8);
+    cudaError_t ce = device_malloc((void**)&tab, count * 8);
     if (ce != cudaSuccess) return cuda_fail(ce, "fold table");
     int rc = small_powers(field, H.inv(g[0]), H.to_tw(half_inv), tab, count, c.stream);
     if (rc) {
@@ -1098,6 +1098,8 @@ int small_fri_fold(int field, const uint64_t* d_layer, uint32_t log_n, const uin
   if (ce != cudaSuccess) return cuda_fail(ce, "fri fold");
   return ZNTT_OK;
 }
+
+void small_drop_idle() { small_evict(small_state().idle_budget + 1); }
 
 void small_shutdown() {
   for (auto& kv : small_fold_tables())

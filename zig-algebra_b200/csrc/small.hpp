@@ -49,6 +49,8 @@ int fri_commit_layer(int field, const uint64_t* d_layer, uint32_t log_n, uint8_t
 int fri_fold_commit(int field, const uint64_t* d_layer, uint32_t log_n, const uint64_t alpha[4], uint64_t* d_out,
                     uint32_t log_table, uint8_t* d_nodes, uint8_t* root_out, void* stream, bool settle);
 void small_shutdown();
+// Frees the tables without a user.
+void small_drop_idle();
 // FRI fold tables of the 256-bit fields (fri.cu).
 void fri_shutdown();
 
