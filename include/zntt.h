@@ -194,7 +194,8 @@ typedef struct zntt_job {
 typedef struct zntt_batch zntt_batch;
 
 /* Plans the jobs (shape: a pass shape index, or -1 for the library's batch
- * shape, 2^9-element tiles at 7 CTAs per SM) and
+ * shape, 2^9-element tiles at 7 CTAs per SM; jobs on tables of 2^29 elements and
+ * more have a shape of their own) and
  * uploads the work queue; buffers stay owned by the caller and must outlive
  * the batch. */
 int zntt_batch_create(int field, const zntt_job* jobs, size_t n_jobs, int shape, zntt_batch** out);

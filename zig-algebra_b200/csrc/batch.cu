@@ -37,7 +37,7 @@ __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
 
 // FULL: every pass of the batch has whole tiles (k + c == LOG_TILE), so the
 // tile runs without bound checks, as the plain pass kernel does for such passes.
-template <class F, int LOG_TILE, int THREADS, int MINB, bool EXT, bool FULL>
+template <class F, int LOG_TILE, int THREADS, int MINB, bool EXT, bool FULL, bool STRIDED = false>
 __global__ void __launch_bounds__(THREADS, MINB)
     batch_kernel(const BatchPass* __restrict__ passes, const BatchItem* __restrict__ items, uint32_t n_items,
                  uint32_t* ctl, uint32_t spin_limit) {
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
     // 520-transform batch 2.94 -> 2.80 ms, 64 coset extensions 16.7 -> 16.3 ms,
     // B200).
     const PassParams pp = s_pp;
-    ntt_tile<F, LOG_TILE, THREADS, true, EXT, FULL>(pp, item.tile, sm);
+    ntt_tile<F, LOG_TILE, THREADS, true, EXT, FULL, true, STRIDED>(pp, item.tile, sm);
     __syncthreads();  // every thread's stores are issued and its shared-memory reads done
     if (threadIdx.x == 0) {
       __threadfence();  // ... and, through the barrier, visible device-wide before the count
@@ -179,6 +179,15 @@ static void launch_batch_shape(bool ext, bool full, const BatchPass* passes, con
   }
 }
 
+// A batch with a strided table among its jobs' (the others may be flat).
+template <class F>
+static void launch_batch_strided(const BatchPass* passes, const BatchItem* items, uint32_t n_items, uint32_t* ctl,
+                                 uint32_t spin_limit, int grid, cudaStream_t st) {
+  constexpr PassShape S = kShapes[kStridedShape];
+  batch_kernel<F, S.log_tile, S.threads, S.min_blocks, true, false, true>
+      <<<grid, S.threads, shape_smem_bytes(kStridedShape), st>>>(passes, items, n_items, ctl, spin_limit);
+}
+
 template <class F>
 static void launch_batch_typed(int shape, bool ext, bool full, const BatchPass* passes, const BatchItem* items,
                                uint32_t n_items, uint32_t* ctl, uint32_t spin_limit, int grid, cudaStream_t st) {
@@ -191,8 +200,15 @@ static void launch_batch_typed(int shape, bool ext, bool full, const BatchPass* 
   }
 }
 
-cudaError_t launch_batch(int field, int shape, bool ext, bool full, const BatchPass* passes, const BatchItem* items,
-                         uint32_t n_items, uint32_t* ctl, uint32_t spin_limit, int grid, cudaStream_t st) {
+cudaError_t launch_batch(int field, int shape, bool ext, bool full, bool strided, const BatchPass* passes,
+                         const BatchItem* items, uint32_t n_items, uint32_t* ctl, uint32_t spin_limit, int grid,
+                         cudaStream_t st) {
+  if (strided) {
+    if (shape != kStridedShape) return cudaErrorInvalidValue;
+    if (field == kBn254Fr) launch_batch_strided<Bn254Fr>(passes, items, n_items, ctl, spin_limit, grid, st);
+    else launch_batch_strided<Bls12381Fr>(passes, items, n_items, ctl, spin_limit, grid, st);
+    return cudaGetLastError();
+  }
   if (field == kBn254Fr)
     launch_batch_typed<Bn254Fr>(shape, ext, full, passes, items, n_items, ctl, spin_limit, grid, st);
   else

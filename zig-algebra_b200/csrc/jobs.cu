@@ -39,7 +39,9 @@ int acquire_coset_tab(int field, uint32_t log_in, const uint64_t* shift, CosetTa
   t->field = field;
   t->log_in = log_in;
   std::memcpy(t->shift, shift, 32);
-  t->bytes = ((size_t)64) << log_in;
+  const bool narrow = narrow_factors(1ull << log_in);
+  t->kind = narrow ? kScaleElements : kScaleFixedTab;
+  t->bytes = (size_t)(narrow ? 32 : 64) << log_in;
   cudaError_t ce = device_malloc((void**)&t->d, t->bytes);
   if (ce != cudaSuccess) {
     delete t;
@@ -57,7 +59,7 @@ int acquire_coset_tab(int field, uint32_t log_in, const uint64_t* shift, CosetTa
     return rc;
   }
   ce = cudaMemcpyAsync(d_pw, pw.data(), pw.size() * 8, cudaMemcpyHostToDevice, st);
-  if (ce == cudaSuccess) ce = launch_powers(field, (const uint4*)d_pw, ninv, t->d, 1ull << log_in, true, st);
+  if (ce == cudaSuccess) ce = launch_powers(field, (const uint4*)d_pw, ninv, t->d, 1ull << log_in, !narrow, st);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
   pool_put(d_pw, pw.size() * 8);
   if (ce != cudaSuccess) {
@@ -104,6 +106,7 @@ static PassParams pass_params(const TwEntry* tw, uint32_t log_n, const PassDesc&
   pp.src = src;
   pp.dst = dst;
   pp.tw = tw->d_table;
+  pp.tw_flat = tw->flat;
   pp.wide = pass_wide(src, dst);
   pp.log_n = log_n;
   pp.S = d.S;
@@ -179,6 +182,7 @@ struct zntt_batch {
   int grid = 0;
   bool ext = false;   // some pass pads or scales by a table
   bool full = false;  // every pass has whole tiles (the kernel runs without bound checks)
+  bool strided = false;  // some job's twiddle table is strided (the shape is kStridedShape then)
   uint32_t spin_limit = ZNTT_BATCH_SPIN_LIMIT;  // x ~0.25-1 us: a stalled dependency gives up after seconds
   std::vector<std::pair<void*, size_t>> scratch;  // pool buffers owned by the batch
   std::vector<CosetTab*> coset_tabs;
@@ -236,7 +240,12 @@ int zntt_batch_create(int field, const zntt_job* jobs, size_t n_jobs, int shape,
   }
   zntt_batch* b = new zntt_batch();
   b->field = field;
-  b->shape = shape >= 0 ? shape : kBatchShape;
+  const auto strided = [](const zntt_twiddles* t) { return t && tw_of(t)->flat < tw_of(t)->log_n; };
+  for (size_t j = 0; j < n_jobs; j++) {
+    const bool lde = jobs[j].kind == ZNTT_JOB_COSET_LDE;
+    b->strided = b->strided || strided(jobs[j].tw) || (lde && strided(jobs[j].tw_in));
+  }
+  b->shape = b->strided ? kStridedShape : shape >= 0 ? shape : kBatchShape;
   cudaStream_t st = c.stream;
 
   std::vector<JobPlan> plans(n_jobs);
@@ -296,7 +305,7 @@ int zntt_batch_create(int field, const zntt_job* jobs, size_t n_jobs, int shape,
       b->scratch.push_back({coef, (size_t)32 << Li});
       const Plan pin = batch_plan(field, Li, b->shape);
       const Plan pout = batch_plan(field, L, b->shape);
-      plan_transform(plans[j], twi, pin, Li, src, (uint4*)coef, (uint4*)coef, true, kScaleFixedTab, ct->d, 1ull << Li,
+      plan_transform(plans[j], twi, pin, Li, src, (uint4*)coef, (uint4*)coef, true, ct->kind, ct->d, 1ull << Li,
                      1ull << Li);
       plan_transform(plans[j], tw, pout, L, (const uint4*)coef, dst, dst, false, kScaleNone, nullptr, 1ull << Li,
                      1ull << L);
@@ -356,8 +365,8 @@ static int enqueue_batch(zntt_batch* b, cudaStream_t st) {
   cudaError_t ce = cudaMemsetAsync(b->d_ctl, 0, b->ctl_words * 4, st);
   if (ce != cudaSuccess) return cuda_fail(ce, "batch reset");
   if (b->items.empty()) return ZNTT_OK;
-  ce = launch_batch(b->field, b->shape, b->ext, b->full, b->d_passes, b->d_items, (uint32_t)b->items.size(), b->d_ctl,
-                    b->spin_limit, b->grid, st);
+  ce = launch_batch(b->field, b->shape, b->ext, b->full, b->strided, b->d_passes, b->d_items,
+                    (uint32_t)b->items.size(), b->d_ctl, b->spin_limit, b->grid, st);
   if (ce != cudaSuccess) return cuda_fail(ce, "batch launch");
   return ZNTT_OK;
 }
@@ -471,7 +480,7 @@ int zntt_coset_lde_device(const zntt_twiddles* tw_in, const zntt_twiddles* tw_ou
   JobPlan jp;
   const Plan pin = tuned_plan(ti->field, ti->log_n);
   const Plan pout = tuned_plan(to->field, to->log_n);
-  plan_transform(jp, ti, pin, ti->log_n, (const uint4*)d_evals, (uint4*)coef, (uint4*)coef, true, kScaleFixedTab, ct->d,
+  plan_transform(jp, ti, pin, ti->log_n, (const uint4*)d_evals, (uint4*)coef, (uint4*)coef, true, ct->kind, ct->d,
                  1ull << ti->log_n, 1ull << ti->log_n);
   plan_transform(jp, to, pout, to->log_n, (const uint4*)coef, (uint4*)d_out, (uint4*)d_out, false, kScaleNone, nullptr,
                  1ull << ti->log_n, 1ull << to->log_n);
@@ -515,6 +524,7 @@ int zntt_coset_lde_columns(const zntt_twiddles* tw_in, const zntt_twiddles* tw_o
 int zntt_autotune(int field, uint32_t log_n_min, uint32_t log_n_max) {
   clear_error();
   if (field != kBn254Fr && field != kBls12381Fr) return set_error(ZNTT_ERR_UNSUPPORTED_FIELD, "unsupported field");
+  static_assert(28 < kStridedLog, "tuned sizes run on flat tables");
   if (log_n_min < 1 || log_n_max > 28 || log_n_min > log_n_max)
     return set_error(ZNTT_ERR_INVALID_ARGUMENT, "autotune range must lie in 1..28");
   Context& c = ctx();

@@ -12,6 +12,7 @@ namespace zntt {
 struct CosetTab {
   int field = 0;
   uint32_t log_in = 0;
+  ScaleKind kind = kScaleFixedTab;  // kScaleElements where the factors are 32-byte elements (narrow_factors)
   uint64_t shift[4] = {0, 0, 0, 0};
   uint4* d = nullptr;
   size_t bytes = 0;

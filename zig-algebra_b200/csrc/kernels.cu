@@ -16,11 +16,11 @@ namespace zntt {
 
 // SCALE: the pass scales its outputs (the inverse's last pass, or an
 // extension pass); the extension variants always include it.
-template <class F, int LOG_TILE, int THREADS, int MINB, bool EXT, bool FULL, bool SCALE>
+template <class F, int LOG_TILE, int THREADS, int MINB, bool EXT, bool FULL, bool SCALE, bool STRIDED = false>
 __global__ void __launch_bounds__(THREADS, MINB) ntt_pass_kernel(PassParams pp) {
   extern __shared__ uint4 sm[];
   pass_wait_input();
-  ntt_tile<F, LOG_TILE, THREADS, false, EXT, FULL, SCALE>(pp, blockIdx.x, sm);
+  ntt_tile<F, LOG_TILE, THREADS, false, EXT, FULL, SCALE, STRIDED>(pp, blockIdx.x, sm);
 }
 
 template <class F, int LOG_TILE, int THREADS, int MINB>
@@ -123,8 +123,22 @@ static void launch_pass_typed(int shape, bool ext, const PassParams& pp, dim3 gr
   }
 }
 
+// A pass on a strided table: these transforms' passes all have whole tiles.
+template <class F>
+static void launch_strided(const PassParams& pp, dim3 grid, cudaStream_t st) {
+  constexpr PassShape S = kShapes[kStridedShape];
+  launch_pass_kernel(ntt_pass_kernel<F, S.log_tile, S.threads, S.min_blocks, true, true, true, true>, S.threads,
+                     shape_smem_bytes(kStridedShape), pp, grid, st);
+}
+
 cudaError_t launch_ntt_pass(int field, int shape, const PassParams& pp, uint64_t num_tiles, cudaStream_t st) {
   dim3 grid((unsigned)num_tiles);
+  if (pp.tw_flat < pp.log_n) {
+    if (shape != kStridedShape || pp.k + pp.c != (uint32_t)kShapes[kStridedShape].log_tile) return cudaErrorInvalidValue;
+    if (field == kBn254Fr) launch_strided<Bn254Fr>(pp, grid, st);
+    else launch_strided<Bls12381Fr>(pp, grid, st);
+    return cudaGetLastError();
+  }
   const bool ext = pass_needs_ext(pp);
   if (field == kBn254Fr)
     launch_pass_typed<Bn254Fr>(shape, ext, pp, grid, st);
@@ -141,15 +155,15 @@ static int grid_for(uint64_t count) { return (int)std::min<uint64_t>((count + 25
 
 template <class F>
 __global__ void twiddle_table_kernel(const uint4* __restrict__ pw, fe n_inv, uint4* __restrict__ table,
-                                     uint32_t log_n) {
-  const uint64_t total = 1ull << log_n;
+                                     uint32_t log_n, uint32_t flat, uint64_t total) {
   for (uint64_t f = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; f < total;
        f += (uint64_t)gridDim.x * blockDim.x) {
     fe r = n_inv;
-    if (f + 1 < total) {
+    if (f + 1 != 1ull << flat) {
       const uint32_t s = 63 - __clzll(f + 1);           // stage: 2^s - 1 <= f < 2^(s+1) - 1
       const uint64_t j = f + 1 - (1ull << s);
-      const uint64_t e = j << (log_n - 1 - s);           // exponent of root, < 2^(log_n-1)
+      // Exponent of root, < 2^(log_n-1).
+      const uint64_t e = f >> flat ? f - (1ull << flat) : j << (log_n - 1 - s);
       const uint32_t e0 = e & 1023, e1 = (e >> 10) & 1023, e2 = (uint32_t)(e >> 20);
       r = fe_mul<F>(fe_load_nc(pw + 2 * e0), fe_load_nc(pw + 2 * (1024 + e1)));
       r = fe_mul<F>(r, fe_load_nc(pw + 2 * (2048 + e2)));
@@ -159,14 +173,15 @@ __global__ void twiddle_table_kernel(const uint4* __restrict__ pw, fe n_inv, uin
 }
 
 cudaError_t launch_twiddle_table(int field, const uint4* d_pw, const uint64_t* n_inv, uint4* d_table, uint32_t log_n,
-                                 cudaStream_t st) {
+                                 uint32_t flat, cudaStream_t st) {
   fe ni;
   std::memcpy(ni.v, n_inv, 32);
-  const int blocks = grid_for(1ull << log_n);
+  const uint64_t total = table_entries(log_n, flat);
+  const int blocks = grid_for(total);
   if (field == kBn254Fr)
-    twiddle_table_kernel<Bn254Fr><<<blocks, 256, 0, st>>>(d_pw, ni, d_table, log_n);
+    twiddle_table_kernel<Bn254Fr><<<blocks, 256, 0, st>>>(d_pw, ni, d_table, log_n, flat, total);
   else
-    twiddle_table_kernel<Bls12381Fr><<<blocks, 256, 0, st>>>(d_pw, ni, d_table, log_n);
+    twiddle_table_kernel<Bls12381Fr><<<blocks, 256, 0, st>>>(d_pw, ni, d_table, log_n, flat, total);
   return cudaGetLastError();
 }
 
@@ -199,18 +214,20 @@ cudaError_t launch_twiddle_pairs(int field, const uint4* d_entries, const uint64
 }
 
 template <class F>
-__global__ void pair_entries_kernel(const uint4* __restrict__ pairs, uint4* __restrict__ entries, uint64_t count) {
+__global__ void pair_entries_kernel(const uint4* __restrict__ pairs, uint32_t step, uint4* __restrict__ entries,
+                                    uint64_t count) {
   for (uint64_t f = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; f < count;
        f += (uint64_t)gridDim.x * blockDim.x)
-    fe_store(entries + 2 * f, pair_entry<F>(ld_fe32(pairs + 4 * f + 2)));
+    fe_store(entries + 2 * f, pair_entry<F>(ld_fe32(pairs + ((4 * f) << step) + 2)));
 }
 
-cudaError_t launch_pair_entries(int field, const uint4* d_pairs, uint4* d_entries, uint64_t count, cudaStream_t st) {
+cudaError_t launch_pair_entries(int field, const uint4* d_pairs, uint32_t step, uint4* d_entries, uint64_t count,
+                                cudaStream_t st) {
   if (count == 0) return cudaSuccess;
   if (field == kBn254Fr)
-    pair_entries_kernel<Bn254Fr><<<grid_for(count), 256, 0, st>>>(d_pairs, d_entries, count);
+    pair_entries_kernel<Bn254Fr><<<grid_for(count), 256, 0, st>>>(d_pairs, step, d_entries, count);
   else
-    pair_entries_kernel<Bls12381Fr><<<grid_for(count), 256, 0, st>>>(d_pairs, d_entries, count);
+    pair_entries_kernel<Bls12381Fr><<<grid_for(count), 256, 0, st>>>(d_pairs, step, d_entries, count);
   return cudaGetLastError();
 }
 

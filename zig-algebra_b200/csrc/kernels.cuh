@@ -43,6 +43,7 @@ struct PassParams {
   const uint4* scale_tab;  // the factor, or the table whose entry q multiplies output position q
   uint64_t src_len;   // first pass: natural input index >= src_len reads as zero (zero padding)
   uint64_t dst_len;   // output positions >= dst_len are not stored
+  uint32_t tw_flat;   // stages from here on share the last one's table entries (log_n but in strided tables)
 };
 
 // Pass kernel shapes.  Each shape is a compiled kernel: a tile of 2^log_tile
@@ -75,6 +76,25 @@ constexpr uint32_t kRadix2MaxLog = 16;
 // 2.26, the 6-CTA 2^9 tile 2.27, the 2^10 tile 2.37, the 2^8 tile 2.42; 64 coset
 // extensions 2^18 -> 2^20 (BLS12-381-Fr) 11.9 / 11.9 / 12.1 / 12.6 / 13.0 (B200).
 constexpr int kBatchShape = 4;
+// Root-derived tables from this size on are strided: the last stage's 2^(log_n - 1)
+// entries also serve the five stages before it, whose entries are every second, every
+// fourth, ... of them, and only the stages below have entries of their own.  That is 33
+// bytes an element instead of 64, about what 32-byte entries took: a BLS12-381-Fr
+// extension 2^29 -> 2^30 takes 130 GiB with its tables, 192 with flat ones.  The passes
+// on strided tables have their own kernels on one shape (2^29 forward 109.8 ms, 109.9 on
+// a flat table; B200): below, the tables stay flat and the hot kernels without the stride,
+// which cost them 0.3 to 0.9%.
+constexpr uint32_t kStridedLog = 29;
+constexpr uint32_t kStridedStages = 6;
+constexpr int kStridedShape = 2;
+inline uint32_t table_flat_stages(uint32_t log_n) { return log_n < kStridedLog ? log_n : log_n - kStridedStages; }
+// Entries of a table, 1/n among them (entry 2^flat - 1).
+inline uint64_t table_entries(uint32_t log_n, uint32_t flat) {
+  return flat == log_n ? 1ull << log_n : (1ull << flat) + (1ull << (log_n - 1));
+}
+// Tables of one factor per element (an extension's, a fold's) of 2^29 entries and more
+// hold 32-byte elements, whose product is a Montgomery product, for the same reason.
+inline bool narrow_factors(uint64_t count) { return count >= 1ull << kStridedLog; }
 constexpr int kLogTile = 11;  // the largest tile of any shape
 constexpr int kDefaultShape = 0;
 
@@ -112,7 +132,8 @@ struct BatchItem {
 // Every wait for a finished pass spins at most `spin_limit` rounds of ~1 us,
 // then raises the error flag; every CTA stops at the next item once it is set.
 // `full`: every pass has whole tiles (batch_all_full), so no bound checks.
-cudaError_t launch_batch(int field, int shape, bool ext, bool full, const BatchPass* passes, const BatchItem* items,
+// strided: some pass's twiddle table is strided (kStridedShape only).
+cudaError_t launch_batch(int field, int shape, bool ext, bool full, bool strided, const BatchPass* passes, const BatchItem* items,
                          uint32_t n_items, uint32_t* ctl, uint32_t spin_limit, int grid, cudaStream_t st);
 // True when every pass's tile is the shape's whole tile (k + c == log_tile).
 inline bool batch_all_full(int shape, const BatchPass* passes, size_t n) {
@@ -122,18 +143,20 @@ inline bool batch_all_full(int shape, const BatchPass* passes, size_t n) {
 }
 int batch_grid(int field, int shape, bool ext);
 
-// Flat zig-ntt twiddle table for one (field, log_n, root), as fixed factors:
-// entry 2^s - 1 + j of stage s is root^(j * 2^(log_n-1-s)), and the last entry
-// (2^log_n - 1) is 1/n, given in Montgomery form.  The powers are assembled from three
+// zig-ntt twiddle table for one (field, log_n, root), as fixed factors: entry
+// 2^s - 1 + j of stage s < flat is root^(j * 2^(log_n-1-s)), entry 2^flat - 1 is 1/n,
+// given in Montgomery form, and in a strided table (flat < log_n) entry 2^flat + j is
+// root^j, j < 2^(log_n - 1).  The powers are assembled from three
 // small host-made tables: pw[0][i] = root^i, pw[1][i] = root^(1024 i),
 // pw[2][i] = root^(2^20 i), i < 1024 (each 1024 x 32 bytes, contiguous).
 cudaError_t launch_twiddle_table(int field, const uint4* d_pw, const uint64_t* n_inv, uint4* d_table, uint32_t log_n,
-                                 cudaStream_t st);
-// The same from the table's 2^log_n - 1 entries in Montgomery form.
+                                 uint32_t flat, cudaStream_t st);
+// A flat table from its 2^log_n - 1 entries in Montgomery form.
 cudaError_t launch_twiddle_pairs(int field, const uint4* d_entries, const uint64_t* n_inv, uint4* d_table,
                                  uint32_t log_n, cudaStream_t st);
-// `count` fixed factors from d_pairs on, back in Montgomery form.
-cudaError_t launch_pair_entries(int field, const uint4* d_pairs, uint4* d_entries, uint64_t count, cudaStream_t st);
+// `count` fixed factors from d_pairs on, every 2^step-th one, back in Montgomery form.
+cudaError_t launch_pair_entries(int field, const uint4* d_pairs, uint32_t step, uint4* d_entries, uint64_t count,
+                                cudaStream_t st);
 
 // out[i] = c * base^i for i < count (count <= 2^30), from the three power
 // tables of `base` laid out as for launch_twiddle_table; `pairs`: as fixed factors.

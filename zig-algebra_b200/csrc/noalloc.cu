@@ -36,6 +36,7 @@
 namespace zntt {
 
 constexpr uint32_t kNoAllocMaxLog = 18;
+static_assert(kNoAllocMaxLog < kStridedLog, "flat tables");
 static __device__ __align__(256) uint4 g_noalloc_scratch[2u << kNoAllocMaxLog];
 
 constexpr int kMaxDevices = 64;
@@ -109,6 +110,7 @@ extern "C" int zntt_ntt_device_inplace_noalloc(const zntt_twiddles* tw, uint64_t
     pp.src = first ? data : scratch;
     pp.dst = (np == 1 || last) ? data : scratch;
     pp.tw = e->d_table;
+    pp.tw_flat = e->flat;
     pp.wide = pass_wide(pp.src, pp.dst);
     pp.log_n = log_n;
     pp.S = passes[p].S;

@@ -101,13 +101,14 @@ __device__ __forceinline__ void pass_wait_input() { asm volatile("griddepcontrol
 // thread needs a bound check; without the checks the pass runs about 5% faster
 // (2^24 BN254-Fr, B200).  SCALE compiles the output scaling (the inverse's
 // 1/n, the extension's factor table); a pass launched without it must not ask
-// for scaling (pp.scale == 0).
+// for scaling (pp.scale == 0).  STRIDED: the twiddle table may be a strided one.
 //
 // The first stages read their elements straight from global memory and the last
 // ones write theirs there (an element is one 32-byte sector, so a thread's own
 // element moves as efficiently as a coalesced row); shared memory only carries
 // the exchanges between stage pairs.
-template <class F, int LOG_TILE, int THREADS, bool COHERENT, bool EXT, bool FULL = false, bool SCALE = true>
+template <class F, int LOG_TILE, int THREADS, bool COHERENT, bool EXT, bool FULL = false, bool SCALE = true,
+          bool STRIDED = false>
 struct TilePass {
   static constexpr uint32_t TILE_MAX = 1u << LOG_TILE;
   const PassParams& pp;
@@ -172,6 +173,21 @@ struct TilePass {
     if (!EXT || g < pp.dst_len) store_data(pp.dst + ((uint64_t)g << 1), y, wide);
   }
 
+  // The table entries of the stage with `half` butterflies, and the place of its entry
+  // idx among them (strided: below 2^(log_n - 1)).
+  __device__ __forceinline__ const uint4* stage_entries(uint32_t half) const {
+    if constexpr (STRIDED) {
+      if (half >> pp.tw_flat) return tw + (4ull << pp.tw_flat);
+    }
+    return tw + 4ull * (half - 1);
+  }
+  __device__ __forceinline__ uint32_t entry(uint32_t half, uint32_t idx) const {
+    if constexpr (STRIDED) {
+      if (half >> pp.tw_flat) return idx << (pp.log_n - 32 + __clz(half));
+    }
+    return idx;
+  }
+
   // Stages i and i+1 on four elements in registers (rows t0 + {0, h, 2h, 3h}).
   // With u, v -> u + t, u - t, t = tw[j] v, the inverse (inttWithTwiddles: factor
   // one for j = 0, else -tw[2^(s-1) - j]) is the same butterfly with the two
@@ -183,8 +199,8 @@ struct TilePass {
     const uint32_t h = IN ? 1u : 1u << (i - 1);
     const uint32_t half1 = 1u << (S + i - 1);  // stage S+i
     const uint32_t half2 = half1 << 1;         // stage S+i+1
-    const uint4* stw1 = tw + 4ull * (half1 - 1);
-    const uint4* stw2 = tw + 4ull * (half2 - 1);
+    const uint4* stw1 = stage_entries(half1);
+    const uint4* stw2 = stage_entries(half2);
     const uint32_t col = ga & (C - 1), g = ga >> c;
     const uint32_t j = g & (h - 1);
     const uint32_t t0 = IN ? g << 2 : ((g >> (i - 1)) << (i + 1)) | j;
@@ -199,10 +215,10 @@ struct TilePass {
     }
     const bool mul = !(jg1 == 0 && unit0);
     const bool swap = inverse && jg1 != 0;  // first-stage results exchanged
-    const uint32_t i1 = inverse ? half1 - jg1 : jg1;
+    const uint32_t i1 = entry(half1, inverse ? half1 - jg1 : jg1);
     // Second stage: the sums' pair and the differences' pair.
     const uint32_t jp = swap ? jg3 : jg1, jm = swap ? jg1 : jg3;
-    const uint32_t ip = inverse ? half2 - jp : jp, im = inverse ? half2 - jm : jm;
+    const uint32_t ip = entry(half2, inverse ? half2 - jp : jp), im = entry(half2, inverse ? half2 - jm : jm);
     fe x0, x1, x2, x3;
     if constexpr (IN) {
       const uint32_t rv = first ? rev_bits(t0, k) : 0;  // t0 is a multiple of 4
@@ -259,7 +275,7 @@ struct TilePass {
   __device__ __forceinline__ void single(uint32_t ga, bool last) const {
     const uint32_t h = 1u << (k - 1);
     const uint32_t half = 1u << (S + k - 1);  // stage S+k
-    const uint4* stw = tw + 4ull * (half - 1);
+    const uint4* stw = stage_entries(half);
     const uint32_t col = ga & (C - 1), j = ga >> c;
     const uint32_t jg = first ? j : (j << S) + m0 + col;
     const bool swap = inverse && jg != 0;
@@ -271,7 +287,7 @@ struct TilePass {
     } else {
       v = sm_load<TILE_MAX>(sm, e0 + (h << c));
     }
-    const fe t = times_factor<F>(!(jg == 0 && unit0), stw, inverse ? half - jg : jg, v);
+    const fe t = times_factor<F>(!(jg == 0 && unit0), stw, entry(half, inverse ? half - jg : jg), v);
     if constexpr (!IN) u = sm_load<TILE_MAX>(sm, e0);
     fe_butterfly<F>(fe_weak<F>(u), t, y, z);
     const uint32_t base = out_base(col);
@@ -422,9 +438,10 @@ __device__ __forceinline__ void ntt_tile_radix2(const PassParams& pp, uint32_t b
   }
 }
 
-template <class F, int LOG_TILE, int THREADS, bool COHERENT, bool EXT, bool FULL = false, bool SCALE = true>
+template <class F, int LOG_TILE, int THREADS, bool COHERENT, bool EXT, bool FULL = false, bool SCALE = true,
+          bool STRIDED = false>
 __device__ __forceinline__ void ntt_tile(const PassParams& pp, uint32_t blk, uint4* sm) {
-  TilePass<F, LOG_TILE, THREADS, COHERENT, EXT, FULL, SCALE>(pp, blk, sm).run();
+  TilePass<F, LOG_TILE, THREADS, COHERENT, EXT, FULL, SCALE, STRIDED>(pp, blk, sm).run();
 }
 
 }  // namespace zntt

@@ -244,6 +244,7 @@ Plan one_pass_plan(uint32_t log_n) {
 }
 
 Plan tuned_plan(int field, uint32_t log_n) {
+  if (log_n >= kStridedLog) return make_plan(log_n, kStridedShape, kShapes[kStridedShape].log_tile - 1);
   const TuneEntry* best = nullptr;
   for (const TuneEntry& t : ctx().tune)
     if (t.field == field && t.log_n == log_n && (!best || t.us < best->us)) best = &t;
@@ -272,6 +273,7 @@ int run_plan(int field, const TwEntry* tw, const Plan& plan, uint32_t log_n, con
     pp.src = cur_src;
     pp.dst = last ? d_dst : mid;
     pp.tw = tw->d_table;
+    pp.tw_flat = tw->flat;
     pp.wide = pass_wide(pp.src, pp.dst);
     pp.log_n = log_n;
     pp.S = d.S;
@@ -317,8 +319,6 @@ static std::string table_key(int field, uint32_t log_n, const uint64_t* root) {
                 (unsigned long long)root[0]);
   return buf;
 }
-
-static size_t table_bytes(uint32_t log_n) { return (size_t)64 << log_n; }
 
 static void free_entry(TwEntry* e) {
   Context& c = ctx();
@@ -391,7 +391,8 @@ static int fill_table(TwEntry* e, cudaStream_t st) {
   ZCHECK(cudaMemcpyAsync(d_pw.p, pw.data(), pw.size() * 8, cudaMemcpyHostToDevice, st), "twiddle powers upload");
   uint64_t ninv[4];
   n_inverse(e->field, e->log_n, ninv);
-  ZCHECK(launch_twiddle_table(e->field, (const uint4*)d_pw.p, ninv, e->d_table, e->log_n, st), "twiddle kernel");
+  ZCHECK(launch_twiddle_table(e->field, (const uint4*)d_pw.p, ninv, e->d_table, e->log_n, e->flat, st),
+         "twiddle kernel");
   ZCHECK(cudaStreamSynchronize(st), "twiddle kernel");
   return ZNTT_OK;
 }
@@ -411,7 +412,8 @@ int acquire_table(int field, uint32_t log_n, const uint64_t* root, TwEntry** out
   e->field = field;
   e->log_n = log_n;
   std::memcpy(e->root, root, 32);
-  e->bytes = table_bytes(log_n);
+  e->flat = table_flat_stages(log_n);
+  e->bytes = table_entries(log_n, e->flat) * 64;
   evict_tables(e->bytes);
   cudaError_t ce = device_malloc((void**)&e->d_table, e->bytes);
   if (ce != cudaSuccess) {
@@ -455,7 +457,8 @@ static int upload_foreign_table(int field, uint32_t log_n, const zntt_stage* sta
   e->field = field;
   e->log_n = log_n;
   e->foreign = true;
-  e->bytes = table_bytes(log_n);
+  e->flat = log_n;
+  e->bytes = table_entries(log_n, e->flat) * 64;
   cudaError_t ce = device_malloc((void**)&e->d_table, e->bytes);
   if (ce != cudaSuccess) {
     delete e;
@@ -809,7 +812,8 @@ int zntt_precompute_twiddles(int field, size_t log_n, const uint64_t root[4], ui
   // The caller's table holds the entries in Montgomery form: made from the
   // device's fixed factors in pieces of at most 2^22 entries, each one launch and
   // then a copy per stage it holds (a launch per stage: 2^10 214 us, 166 so; B200).
-  const size_t total = ((size_t)1 << log_n) - 1, piece = (size_t)1 << std::min<size_t>(22, log_n);
+  const uint32_t flat = tw->flat;
+  const size_t total = ((size_t)1 << flat) - 1, piece = (size_t)1 << std::min<size_t>(22, log_n);
   PoolBuf d_entries;
   rc = d_entries.get(piece * 32);
   if (rc) {
@@ -819,12 +823,22 @@ int zntt_precompute_twiddles(int field, size_t log_n, const uint64_t root[4], ui
   cudaError_t e = cudaSuccess;
   for (size_t at = 0; at < total && e == cudaSuccess; at += piece) {
     const size_t end = std::min(at + piece, total);
-    e = launch_pair_entries(field, tw->d_table + 4 * at, (uint4*)d_entries.p, end - at, c.stream);
-    for (size_t s = 0; s < log_n && e == cudaSuccess; s++) {
+    e = launch_pair_entries(field, tw->d_table + 4 * at, 0, (uint4*)d_entries.p, end - at, c.stream);
+    for (size_t s = 0; s < flat && e == cudaSuccess; s++) {
       const size_t first = ((size_t)1 << s) - 1, lo = std::max(at, first), hi = std::min(end, 2 * first + 1);
       if (lo < hi)
         e = cudaMemcpyAsync(stage_out[s] + 4 * (lo - first), (const uint4*)d_entries.p + 2 * (lo - at), (hi - lo) * 32,
                             cudaMemcpyDeviceToHost, c.stream);
+    }
+  }
+  for (size_t s = flat; s < log_n && e == cudaSuccess; s++) {  // a strided table's other stages
+    const uint32_t step = (uint32_t)(log_n - 1 - s);
+    for (size_t at = 0; at < (size_t)1 << s && e == cudaSuccess; at += piece) {
+      const size_t m = std::min(piece, ((size_t)1 << s) - at);
+      e = launch_pair_entries(field, tw->d_table + 4 * (((size_t)1 << flat) + (at << step)), step, (uint4*)d_entries.p, m,
+                              c.stream);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(stage_out[s] + 4 * at, d_entries.p, m * 32, cudaMemcpyDeviceToHost, c.stream);
     }
   }
   const cudaError_t se = cudaStreamSynchronize(c.stream);

@@ -15,19 +15,21 @@
 
 namespace zntt {
 
-// A device twiddle table in zig-ntt's flat layout (stage s at entry 2^s - 1), as
-// fixed factors of 64 bytes (shoup.cuh), and 1/n as its last entry.
+// A device twiddle table as fixed factors of 64 bytes (shoup.cuh): zig-ntt's flat layout
+// (stage s at entry 2^s - 1) for the stages below `flat`, then 1/n, and in a strided
+// table (kernels.cuh) the last stage's entries, which the stages from `flat` on share.
 struct TwEntry {
   int field = 0;
   uint32_t log_n = 0;
   uint64_t root[4] = {0, 0, 0, 0};  // Montgomery form; the key of root-derived tables
-  uint4* d_table = nullptr;         // 2^log_n entries of 4 uint4
+  uint32_t flat = 0;                // log_n but in strided tables
+  uint4* d_table = nullptr;         // table_entries(log_n, flat) entries of 4 uint4
   size_t bytes = 0;
   int refs = 0;                     // handles + registrations holding it
   bool tw0_one = true;              // every stage's entry 0 equals one
   bool foreign = false;             // uploaded from a caller's table, not derived from a root
   uint64_t last_use = 0;
-  const uint4* n_inv() const { return d_table + 4 * (((size_t)1 << log_n) - 1); }
+  const uint4* n_inv() const { return d_table + 4 * (((size_t)1 << flat) - 1); }
 };
 
 // A host table made by zntt_precompute_twiddles, recognised again by its stage

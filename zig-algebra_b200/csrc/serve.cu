@@ -310,7 +310,7 @@ static bool launch_into(zntt_server* s, Slot& sl) {
       const Plan pi = batch_plan(field, r.log_in, shape);
       const Plan po = batch_plan(field, r.log_n, shape);
       plan_transform(plans[j], twi, pi, r.log_in, (const uint4*)q.d_in, (uint4*)q.d_coef, (uint4*)q.d_coef, true,
-                     kScaleFixedTab, q.ct->d, 1ull << r.log_in, 1ull << r.log_in);
+                     q.ct->kind, q.ct->d, 1ull << r.log_in, 1ull << r.log_in);
       plan_transform(plans[j], tw, po, r.log_n, (const uint4*)q.d_coef, (uint4*)q.d_out, (uint4*)q.d_out, false,
                      kScaleNone, nullptr, 1ull << r.log_in, 1ull << r.log_n);
     }
@@ -362,7 +362,7 @@ static bool launch_into(zntt_server* s, Slot& sl) {
     if (ce == cudaSuccess) {
       const int grid = std::max(1, std::min<int>(ext ? s->grid_ext : s->grid_plain, (int)ni));
       const bool full = batch_all_full(kBatchShape, sl.h_passes, np);
-      ce = launch_batch(field, kBatchShape, ext, full, sl.d_passes, sl.d_items, ni, sl.d_ctl, ZNTT_BATCH_SPIN_LIMIT,
+      ce = launch_batch(field, kBatchShape, ext, full, false, sl.d_passes, sl.d_items, ni, sl.d_ctl, ZNTT_BATCH_SPIN_LIMIT,
                         grid, st);
     }
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(sl.h_flag, sl.d_ctl + 1, 4, cudaMemcpyDeviceToHost, st);
@@ -492,6 +492,7 @@ int zntt_server_submit(zntt_server* s, const zntt_request* r) {
   clear_error();
   if (!s || !r || !r->h_in || !r->h_out) return set_error(ZNTT_ERR_INVALID_ARGUMENT, "null pointer");
   const bool lde = r->kind == ZNTT_JOB_COSET_LDE;
+  static_assert(28 < kStridedLog, "requests run on flat tables");
   if ((r->kind != ZNTT_JOB_NTT && !lde) || r->log_n > 28 || (lde && r->log_in > r->log_n) ||
       (!lde && r->mode != ZNTT_FORWARD && r->mode != ZNTT_INVERSE))
     return set_error(ZNTT_ERR_INVALID_ARGUMENT, "malformed request");
