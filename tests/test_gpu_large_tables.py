@@ -131,3 +131,71 @@ def test_an_extension_of_2p29_fits(fresh):
         s = sum(e * pow(wi, i, P) * pow(x - pow(wi, i, P), -1, P) for i, e in zip(at, es))
         want.append((pow(x, n, P) - 1) * pow(n, -1, P) * s % P)
     assert _get(out, ks) == want
+
+
+def _fold_inputs(log_n):
+    layer = O.random_elements(FID, 300 + log_n, 1 << log_n)
+    return layer, O.random_elements(FID, 400 + log_n, 1)[0]
+
+
+@pytest.mark.parametrize("log_n", [1, 2, 5, 9, 13])
+def test_folds_with_a_large_table(fresh, log_n):
+    """Folds (alone, and with the commitment of their result) by the table of a 2^30 domain, which
+    takes 16 GiB: 32 bytes an entry."""
+    import torch
+    z, log_table = fresh, 30
+    F, half = z.BLS12_381_FR, 1 << (log_n - 1)
+    _need(20)
+    layer, alpha = _fold_inputs(log_n)
+    want = O.fri_fold(FID, layer, log_n, alpha)
+    x = torch.from_numpy(layer.view(np.int64).reshape(-1).copy()).cuda()
+    y = torch.zeros(4 * half, dtype=torch.int64, device="cuda")
+    nodes = torch.zeros(32 * half, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    z.fri_fold(F, x.data_ptr(), log_n, alpha, y.data_ptr(), log_table=log_table)
+    torch.cuda.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] < 17 * GIB
+    assert np.array_equal(y.cpu().numpy().view(np.uint64).reshape(-1, 4), want)
+    if log_n < 2:
+        return
+    y.zero_()
+    torch.cuda.synchronize()
+    root = z.fri_fold_commit(F, x.data_ptr(), log_n, alpha, y.data_ptr(), nodes.data_ptr(), log_table=log_table)
+    torch.cuda.synchronize()
+    assert np.array_equal(y.cpu().numpy().view(np.uint64).reshape(-1, 4), want)
+    tree = O.fri_commit_layer(FID, want, log_n - 1)
+    assert root == bytes(bytearray(np.asarray(tree[1]).view(np.uint8)))
+    assert np.array_equal(nodes.cpu().numpy(), np.asarray(tree).view(np.uint8).reshape(-1))
+
+
+def test_a_fold_and_commitment_of_2p31_fits(fresh):
+    """A layer of 2^31 folded and committed: 64 GiB in, 32 out, 32 of nodes and 32 of factors."""
+    import torch
+    z, log_n = fresh, 31
+    F, n = z.BLS12_381_FR, 1 << log_n
+    _need(163)
+    half = n // 2
+    at = _samples(half, 7)
+    lo, hi = [3 * i + 1 for i in range(len(at))], [P - 5 * i for i in range(len(at))]
+    x = torch.zeros(4 * n, dtype=torch.int64, device="cuda")
+    y = torch.empty(4 * half, dtype=torch.int64, device="cuda")
+    nodes = torch.empty(32 * half, dtype=torch.uint8, device="cuda")
+    _put(x, at, lo)
+    _put(x, [j + half for j in at], hi)
+    alpha = 1 << 77
+    torch.cuda.synchronize()
+    root = z.fri_fold_commit(F, x.data_ptr(), log_n, z.to_montgomery(F, alpha), y.data_ptr(), nodes.data_ptr())
+    torch.cuda.synchronize()
+    g = pow(_root(32), 2, P)
+    got = dict(zip(at, _get(y, at)))
+    for j, a, b in zip(at, lo, hi):
+        assert got[j] == ((a + b) + alpha * (a - b) * pow(g, -j, P)) * pow(2, -1, P) % P, j
+    assert root == bytes(bytearray(nodes[32:64].cpu().numpy()))
+    # Leaf j hashes values j and j + half / 2; a parent its two children.
+    quarter = half // 2
+    pair = _get(y, [1, 1 + quarter])
+    leaf = O.blake3(b"".join(v.to_bytes(32, "little") for v in pair))
+    assert leaf == bytes(bytearray(nodes[32 * (quarter + 1):32 * (quarter + 2)].cpu().numpy()))
+    kids = bytes(bytearray(nodes[64:128].cpu().numpy()))
+    assert O.blake3(kids) == root

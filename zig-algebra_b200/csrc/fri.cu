@@ -28,13 +28,13 @@ namespace {
 // Two products by fixed factors and a halving: 428 multiply-pipe slots against
 // three Montgomery products' 816, and 160 bytes of memory traffic, the two bounds
 // about equal (2^24 -> 2^23 BN254-Fr 0.419 -> 0.237 ms, B200).
-template <class F>
+template <class F, bool NARROW>
 __global__ void fri_fold_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, const uint4* __restrict__ tab,
                                 uint64_t half, uint32_t stride, fe_pair alpha) {
   for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < half;
        j += (uint64_t)gridDim.x * blockDim.x) {
     const fe a = fe_load_nc(in + 2 * j), b = fe_load_nc(in + 2 * (j + half));
-    fe_store(out + 2 * j, fe_fold<F>(a, b, tab + 4 * (j << stride), alpha));
+    fe_store(out + 2 * j, fe_fold<F, NARROW>(a, b, tab, j << stride, alpha));
   }
 }
 
@@ -67,7 +67,8 @@ int powers_device(int field, const uint64_t* base, const uint64_t* c, uint4* out
   return ZNTT_OK;
 }
 
-// The table g^-j / 2 (j < 2^(log_n - 1)) for the subgroup of order 2^log_n, as fixed factors.
+// The table g^-j / 2 (j < 2^(log_n - 1)) for the subgroup of order 2^log_n, as fixed factors
+// (as elements where narrow_factors says so).
 int fold_table(int field, uint32_t log_n, const uint4** out) {
   auto key = std::make_pair(field, log_n);
   auto& tabs = fold_tables();
@@ -85,10 +86,11 @@ int fold_table(int field, uint32_t log_n, const uint4** out) {
   F.inv(two, half_inv);
   FoldTable t;
   const uint64_t count = 1ull << (log_n - 1);
-  t.bytes = count * 64;
+  const bool narrow = narrow_factors(count);
+  t.bytes = count * (narrow ? 32 : 64);
   cudaError_t ce = device_malloc((void**)&t.d, t.bytes);
   if (ce != cudaSuccess) return cuda_fail(ce, "fold table");
-  rc = powers_device(field, ginv, half_inv, t.d, count, true, ctx().stream);
+  rc = powers_device(field, ginv, half_inv, t.d, count, !narrow, ctx().stream);
   if (rc) {
     cudaFree(t.d);
     return rc;
@@ -177,9 +179,11 @@ int zntt_fri_fold_device(int field, const uint64_t* d_layer, uint32_t log_n, con
   const uint4* in = reinterpret_cast<const uint4*>(d_layer);
   uint4* out = reinterpret_cast<uint4*>(d_out);
   if (field == kBn254Fr)
-    fri_fold_kernel<Bn254Fr><<<grid_of(half), 256, 0, st>>>(in, out, tab, half, stride, av);
+    fri_fold_kernel<Bn254Fr, false><<<grid_of(half), 256, 0, st>>>(in, out, tab, half, stride, av);
+  else if (narrow_factors(1ull << (log_table - 1)))
+    fri_fold_kernel<Bls12381Fr, true><<<grid_of(half), 256, 0, st>>>(in, out, tab, half, stride, av);
   else
-    fri_fold_kernel<Bls12381Fr><<<grid_of(half), 256, 0, st>>>(in, out, tab, half, stride, av);
+    fri_fold_kernel<Bls12381Fr, false><<<grid_of(half), 256, 0, st>>>(in, out, tab, half, stride, av);
   cudaError_t ce = cudaGetLastError();
   if (ce != cudaSuccess) return cuda_fail(ce, "fri fold");
   return ZNTT_OK;

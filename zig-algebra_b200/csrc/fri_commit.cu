@@ -87,7 +87,7 @@ struct SmallLeafSource {
 // that hashes it computes both from the previous layer (values m and m + 2h
 // for m = j, j + h: (f_m + f_{m+2h}) / 2 + alpha (f_m - f_{m+2h}) g^-m / 2,
 // the factor from the resident table at stride 2^stride) and stores them.
-template <class F>
+template <class F, bool NARROW>
 struct WideFoldLeafSource {
   const uint4* prev;
   uint4* next;
@@ -97,7 +97,7 @@ struct WideFoldLeafSource {
   fe_pair alpha;
   __device__ __forceinline__ fe fold(uint64_t m) const {
     const fe a = fe_load_nc(prev + 2 * m), b = fe_load_nc(prev + 2 * (m + 2 * h));
-    return fe_fold<F>(a, b, tab + 4 * (m << stride), alpha);
+    return fe_fold<F, NARROW>(a, b, tab, m << stride, alpha);
   }
   __device__ __forceinline__ void get(uint64_t j, uint32_t (&d)[8], uint32_t one) const {
     const fe x = fold(j), y = fold(j + h);
@@ -151,8 +151,8 @@ struct SmallFoldLeafSource {
 // per thread in leaf_kernel rather than two plus their parent per thread in
 // subtree_kernel: 14 rounds from 2^24 BN254-Fr took 3.01 ms that way and 3.19 ms
 // in the subtree kernel.
-template <class F>
-struct OneLeafPerThread<WideFoldLeafSource<F>> {
+template <class F, bool NARROW>
+struct OneLeafPerThread<WideFoldLeafSource<F, NARROW>> {
   static constexpr bool value = true;
 };
 
@@ -313,8 +313,13 @@ int fri_fold_commit(int field, const uint64_t* d_layer, uint32_t log_n, const ui
   uint4* next = reinterpret_cast<uint4*>(d_out);
   const uint4* t4 = reinterpret_cast<const uint4*>(tab);
   if (field == kBn254Fr)
-    return commit_tree(WideFoldLeafSource<Bn254Fr>{prev, next, t4, h, stride, av}, nodes, h, root_out, st, settle, what);
-  return commit_tree(WideFoldLeafSource<Bls12381Fr>{prev, next, t4, h, stride, av}, nodes, h, root_out, st, settle, what);
+    return commit_tree(WideFoldLeafSource<Bn254Fr, false>{prev, next, t4, h, stride, av}, nodes, h, root_out, st, settle,
+                       what);
+  if (narrow_factors(1ull << (log_table - 1)))
+    return commit_tree(WideFoldLeafSource<Bls12381Fr, true>{prev, next, t4, h, stride, av}, nodes, h, root_out, st, settle,
+                       what);
+  return commit_tree(WideFoldLeafSource<Bls12381Fr, false>{prev, next, t4, h, stride, av}, nodes, h, root_out, st, settle,
+                     what);
 }
 
 }  // namespace zntt

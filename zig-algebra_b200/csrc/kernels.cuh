@@ -93,7 +93,8 @@ inline uint64_t table_entries(uint32_t log_n, uint32_t flat) {
   return flat == log_n ? 1ull << log_n : (1ull << flat) + (1ull << (log_n - 1));
 }
 // Tables of one factor per element (an extension's, a fold's) of 2^29 entries and more
-// hold 32-byte elements, whose product is a Montgomery product, for the same reason.
+// hold 32-byte elements, whose product is a Montgomery product, for the same reason (of
+// the two fields only BLS12-381-Fr has folds that large).
 inline bool narrow_factors(uint64_t count) { return count >= 1ull << kStridedLog; }
 constexpr int kLogTile = 11;  // the largest tile of any shape
 constexpr int kDefaultShape = 0;

@@ -449,15 +449,18 @@ __device__ __forceinline__ void fe_butterfly(const fe& u, const fe& t, fe& sum, 
 }
 
 // One FRI fold: (a + b) / 2 + alpha (a - b) / (2 x) for canonical a and b, with the
-// fixed factors 1 / (2 x) (in memory) and alpha.
-template <class F>
-__device__ __forceinline__ fe fe_fold(const fe& a, const fe& b, const uint4* half_inv_x, const fe_pair& alpha) {
+// fixed factors 1 / (2 x) (entry j of a table; NARROW: an element) and alpha.
+template <class F, bool NARROW = false>
+__device__ __forceinline__ fe fe_fold(const fe& a, const fe& b, const uint4* table, uint64_t j, const fe_pair& alpha) {
   const fe even = fe_half<F>(fe_add<F>(a, b));
   fe p;
   p.v[0] = F::P0; p.v[1] = F::P1; p.v[2] = F::P2; p.v[3] = F::P3;
   p.v[4] = F::P4; p.v[5] = F::P5; p.v[6] = F::P6; p.v[7] = F::P7;
   const fe d = fe_sub_raw(fe_add_raw(a, p), b);  // (0, 2p)
-  const fe t = fe_mul_fixed<F>(d, ld_fe32(half_inv_x), ld_fe32(half_inv_x + 2));
+  const uint4* f = table + (NARROW ? 2 : 4) * j;
+  fe t;
+  if constexpr (NARROW) t = fe_mul<F>(fe_load_nc(f), d);
+  else t = fe_mul_fixed<F>(d, ld_fe32(f), ld_fe32(f + 2));
   const fe odd = fe_mul_fixed<F>(t, alpha.w, alpha.q);  // below 2p
   if constexpr (F::kLazy) return fe_canonical<F>(fe_add_raw(even, odd));
   else return fe_add<F>(even, fe_reduce<F>(odd));
