@@ -478,8 +478,11 @@ int zntt_coset_lde_device(const zntt_twiddles* tw_in, const zntt_twiddles* tw_ou
     return rc;
   }
   JobPlan jp;
-  const Plan pin = tuned_plan(ti->field, ti->log_n);
-  const Plan pout = tuned_plan(to->field, to->log_n);
+  Plan pin = tuned_plan(ti->field, ti->log_n);
+  Plan pout = tuned_plan(to->field, to->log_n);
+  // One element: a pass of no stage, which copies and scales.
+  if (ti->log_n == 0) pin = batch_plan(ti->field, 0, pin.shape);
+  if (to->log_n == 0) pout = batch_plan(to->field, 0, pout.shape);
   plan_transform(jp, ti, pin, ti->log_n, (const uint4*)d_evals, (uint4*)coef, (uint4*)coef, true, ct->kind, ct->d,
                  1ull << ti->log_n, 1ull << ti->log_n);
   plan_transform(jp, to, pout, to->log_n, (const uint4*)coef, (uint4*)d_out, (uint4*)d_out, false, kScaleNone, nullptr,
