@@ -52,6 +52,15 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 # BN254-Fr 92 full, 16 low, 4 dot; BLS12-381-Fr 79 full, 14 low, 4 dot (its low
 # limbs' share is shifts and adds).  A Montgomery product takes 272.
 IMAD_PER_MODMUL = {"bn254_fr": 204, "bls12_381_fr": 176}
+
+
+def transform_products(log_n: int, inverse: bool = False) -> float:
+    """Products of one transform: a butterfly each, but none in stage 1 and half of stage 2 (their
+    factors are one, and the kernels skip whole warps of them), and the inverse's 1/n per element."""
+    n = 1 << log_n
+    return (n / 2 * (log_n - 1.5) if log_n >= 2 else 0) + (n if inverse else 0)
+
+
 METRIC = "BN254-Fr NTT elems/s at 2^24"
 
 
@@ -370,7 +379,7 @@ def run_zntt(args, rank, world, local):
     # Roofline: the pass kernel is the only kernel in the timed region.
     imad = z.probe_imad()
     peak_modmul = imad / IMAD_PER_MODMUL["bn254_fr"]
-    modmuls = n / 2 * log_n
+    modmuls = transform_products(log_n)
     achieved = modmuls / (ms_step * 1e-3)
     peaks, peaks_kind = measured_peaks()
     alg_bytes = 2 * n * 32
@@ -402,7 +411,7 @@ def run_zntt(args, rank, world, local):
     line = {
         "metric": metric_name(log_n), "value": value, "unit": "elements/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "u256-mod-r (BN254-Fr, 8x32-bit Montgomery)",
+        "vs_baseline": None, "dtype": "u256-mod-r (BN254-Fr, 8x32-bit limbs, elements in Montgomery form)",
         "data": "synthetic: seeded ChaCha20 randomFieldElement draws generated on the device",
         "config": {"workload": f"bn254_fr_ntt_forward_2^{log_n}", "log_n": log_n, "field": "bn254_fr",
                    "direction": "forward", "twiddles": "precomputed, device-resident",
@@ -512,7 +521,7 @@ def run_size_sweep(z, torch, stream, steps, warmup, imad, seed=66):
     """The single-transform configuration across sizes and directions: BN254-Fr 2^20, 2^22 and
     2^24, forward and inverse (nttWithTwiddles / inttWithTwiddles, libs/ntt/src/root.zig:148-212),
     and BLS12-381-Fr 2^24, with the tables resident.  Each entry: ms per transform, elements/s,
-    the modmul rate ((n/2) log n products, plus n for the inverse's 1/n) over the live
+    the modmul rate (the products made, plus n for the inverse's 1/n) over the live
     multiply-pipe peak, and the algorithmic HBM rate (the vector read and written once,
     2 n 32 bytes) over the measured copy bandwidth."""
     sptr = stream.cuda_stream
@@ -531,7 +540,7 @@ def run_size_sweep(z, torch, stream, steps, warmup, imad, seed=66):
                     for _ in range(warmup):
                         run()
                     ms = time_region(torch, stream, run, steps) / steps
-                    modmuls = n // 2 * L + (n if mode == z.INVERSE else 0)
+                    modmuls = transform_products(L, mode == z.INVERSE)
                     hbm_gbs = 2 * n * 32 / (ms * 1e-3) / 1e9
                     out[f"{F.name} 2^{L} {name}"] = {
                         "ms": ms, "elements_per_s": n / (ms * 1e-3), "modmul_per_s": modmuls / (ms * 1e-3),
@@ -626,7 +635,7 @@ def run_batched_config(z, torch, stream, steps, warmup, seed=33):
         xs.append(x); ys.append(y); ps.append(pl)
         jobs.append({"kind": z.JOB_NTT, "tw": tabs(L), "mode": m, "src": x.data_ptr(), "dst": y.data_ptr()})
     elements = sum(1 << L for L in logs)
-    butterflies = sum((1 << L) // 2 * L for L in logs)
+    products = sum(transform_products(L, m == z.INVERSE) for L, m in zip(logs, modes))
 
     def plain():
         for L, m, x, pl in zip(logs, modes, xs, ps):
@@ -648,7 +657,7 @@ def run_batched_config(z, torch, stream, steps, warmup, seed=33):
         "elements": elements, "jobs": len(logs), "items": info["items"], "grid": info["grid"],
         "shape": info["shape"], "ms_per_batch": ms_b / steps, "value": elements * steps / (ms_b * 1e-3),
         "plain_ms_per_batch": ms_p / steps, "plain_value": elements * steps / (ms_p * 1e-3),
-        "speedup_vs_plain": ms_p / ms_b, "modmul_per_s": butterflies * steps / (ms_b * 1e-3),
+        "speedup_vs_plain": ms_p / ms_b, "modmul_per_s": products * steps / (ms_b * 1e-3),
         "unit": "elements/s", "bit_exact_vs_plain": exact,
     }
 
@@ -685,7 +694,7 @@ def run_lde_config(z, torch, stream, steps, warmup, seed=44, count=64):
         b.status()
     exact = all(torch.equal(o, p) for o, p in zip(outs, pls))
     tabs.close()
-    modmuls = count * ((1 << 17) * 18 + (1 << 18) + (1 << 19) * 20)
+    modmuls = count * (transform_products(18, inverse=True) + transform_products(20))
     return {
         "workload": f"{count} x coset LDE 2^18 -> 2^20 BLS12-381-Fr (g = 5), one persistent launch (CUDA graph)",
         "ms_per_batch": ms_b / steps, "value": count * (1 << 20) * steps / (ms_b * 1e-3), "unit": "output elements/s",
@@ -714,7 +723,7 @@ def run_poly_config(z, torch, stream, steps, warmup, seed=55, cpu_sample=True):
         one()
     ms_one = time_region(torch, stream, one, steps) / steps
     N = 1 << 24
-    modmuls = 3 * (N // 2) * 24 + 2 * N  # three transforms, the pointwise product, n^-1
+    modmuls = 3 * transform_products(24) + 2 * N  # three transforms, the pointwise product, n^-1
 
     m, count = 1 << 14, 64
     pa = torch.empty(count * m * 4, dtype=torch.int64, device="cuda")

@@ -25,7 +25,7 @@ namespace zntt {
 
 namespace {
 
-// Two products by fixed factors and a halving: 428 multiply-pipe slots against
+// Two products by fixed factors and a halving: 408 multiply-pipe slots against
 // three Montgomery products' 816, and 160 bytes of memory traffic, the two bounds
 // about equal (2^24 -> 2^23 BN254-Fr 0.419 -> 0.237 ms, B200).
 template <class F, bool NARROW>

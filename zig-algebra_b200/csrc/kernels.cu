@@ -2,9 +2,11 @@
 //
 // The transform is zig-ntt's radix-2 decimation-in-time network
 // (libs/ntt/src/root.zig:148-212) executed as a few fused passes: each pass
-// stages a tile of the vector in shared memory with coalesced 16-byte global
-// loads, runs several butterfly stages on it, and writes it back.  All
-// arithmetic is exact Montgomery arithmetic from field.cuh.
+// runs several butterfly stages on a tile of the vector, the first on elements
+// read from global memory (32 bytes a load) and the last writing them there, with
+// the exchanges between in shared memory (pass_tile.cuh).  All arithmetic is exact:
+// products by fixed factors (shoup.cuh) in the passes, Montgomery products
+// (field.cuh) where both factors vary and in the making of tables.
 #include <algorithm>
 #include <cstring>
 

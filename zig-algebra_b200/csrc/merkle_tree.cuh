@@ -235,8 +235,8 @@ struct OneLeafPerThread {
   static constexpr bool value = false;
 };
 
-// Leaves, then subtrees of five levels while a level has 512 entries or more,
-// then the rest in one CTA: the launches of a commitment that the caller does
+// Leaves, then subtrees while a level has 512 entries or more (each launch four
+// new levels, five where it makes the leaves too), then the rest in one CTA: the launches of a commitment that the caller does
 // not wait for (it may be captured, or run beside others).
 template <class Src>
 cudaError_t build_tree(const Src& src, uint4* nodes, uint64_t h, cudaStream_t st) {
@@ -260,7 +260,8 @@ cudaError_t build_tree(const Src& src, uint4* nodes, uint64_t h, cudaStream_t st
   return ce;
 }
 
-// Levels of at least this width get launches of their own, one per five levels:
+// Levels of at least this width get launches of their own, one per four new levels
+// (five where the leaves are made too):
 // with as many CTAs the fences and counts of tree_kernel cost more than launches
 // save.  A Goldilocks layer and its root, one launch against this line: 2^18 42.5
 // and 41 us, 2^20 72 and 67, 2^24 560 and 516; below it one launch is the faster

@@ -7,17 +7,18 @@
 // x w - quotient p, whose low 256 bits are all of it (Shoup's method; V. Shoup's
 // NTL, and D. Harvey, "Faster arithmetic for number-theoretic transforms",
 // 2014).  x w and quotient p are needed in their low halves only and x q in its
-// high half, so the three cost 28 + 28 + 43 full 32x32->64 products and 16 low
-// ones where a Montgomery product costs 136 full ones: 214 multiply-pipe slots
-// of a 32-bit multiply-add against 272.  The transforms are bound by that pipe.
+// high half, so the three cost 28 + 28 + 36 full 32x32->64 products, 16 low ones and
+// four dot products of halves and bytes where a Montgomery product costs 136 full
+// ones: 204 multiply-pipe slots of a 32-bit multiply-add against 272 (176 for
+// BLS12-381-Fr, below).  The transforms are bound by that pipe.
 //
 // Which x: any value below 2^256 / 1.03 (lazy fields; below 2p for the others).  The
 // quotient estimate drops the columns of x q below 6, worth less than 2^227, and
 // takes column 6's products x_i q_(6-i) from the 16 top bits of x_i and the 8 top
 // bits of q_(6-i), each low by less than (2^24 + 2^16) 2^224: in all less than
-// 0.0274 2^256, so with q > w 2^256 / p - 1 it is above
-// x w / p - x / 2^256 - 1 - 0.0274 and
-//   0 <= result < (1.0274 + x / 2^256) p.
+// 0.0275 2^256 (seven of them are 0.02745), so with q > w 2^256 / p - 1 it is above
+// x w / p - x / 2^256 - 1 - 0.0275 and
+//   0 <= result < (1.0275 + x / 2^256) p.
 //
 // The factor is the plain value w, not its Montgomery form: x in Montgomery
 // form times w is the product in Montgomery form.  Both parts come out of one
@@ -304,7 +305,7 @@ __device__ __forceinline__ void mul_low_add_hi6(low_acc& s, const fe& x, const f
   s.o[7] += b.v[0] * x.v[5];
 }
 
-// x * w mod p up to a multiple of p, below (1.0274 + x / 2^256) p, for the fixed
+// x * w mod p up to a multiple of p, below (1.0275 + x / 2^256) p, for the fixed
 // factor (w, q).
 //
 // BLS12-381-Fr's low limbs make 28 of the 64 slots of quotient * p shifts and
@@ -406,9 +407,9 @@ static __device__ const __align__(16) Multiples kBnMultiples = make_multiples<Bn
 // which t stays below 1.986 p, so only u needs a bound, and two stages in a row
 // need it once: from u < 1.07 p the first stage's results are below 3.07 p and,
 // as u of the second stage, lead to results below 5.07 p < 2^256.  fe_weak brings a
-// stored value (or a v whose factor is one) below 1.07 p: k = floor of its top
-// byte over 49 (p is 48.39 of those units) is at most x / p and at least
-// x / p - 1.07.
+// stored value (or a v whose factor is one) below 1.07 p: k = its top byte times
+// 84 / 4096 rounded down (p is 48.39 units of that byte, 4096 / 84 is 48.76) is at
+// most x / p and above x / p - 1.07.
 // Other fields (BLS12-381-Fr: 2^256 = 2.21 p) keep values below 2 p, for which t is
 // below 1.934 p: u and t are reduced to [0, p) before each butterfly.
 template <class F>

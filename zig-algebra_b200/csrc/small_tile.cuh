@@ -10,8 +10,8 @@
 // staged by the tile exchanged five times; K and the windows are compile-time
 // constants, and an address serves sixteen elements.  On radix-4 groups staged by
 // the tile a butterfly took 48 instructions (BabyBear) and 77 (Goldilocks); here 16
-// and 45.  BabyBear is bound by memory (2^24: three passes of 268 MB in 0.168 ms,
-// 4.8 TB/s; 0.362 before), Goldilocks by its arithmetic on the ALU and multiply
+// and 45.  BabyBear is bound by memory (2^24: three passes of 268 MB in 0.160 ms,
+// 5.0 TB/s; 0.362 before), Goldilocks by its arithmetic on the ALU and multiply
 // pipes (2^24 0.524 -> 0.382 ms; B200).
 #pragma once
 
